@@ -27,6 +27,8 @@ NVCC_COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-
 SOURCES = {
     "kernels_exact.cu": ["-fmad=false"],
     "engine_exact.cu": ["-fmad=false"],
+    "chip_exact.cu": ["-fmad=false"],
+    "chip_fast.cu": [],
     "control.cu": ["-fmad=false"],
     "output.cu": ["-fmad=false"],
     "mesh_device.cu": [],
@@ -41,7 +43,7 @@ SOURCES = {
     "../unet/csrc/unet_ops.cu": [],
 }
 CXX_SOURCES = {"mesh.cpp": ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off"]}
-HEADERS = [os.path.join(ROOT, "include", "unet.h"), "acs_dev.cuh", "kernels.h", "fast.h", "engine.cuh", "engine_api.h", "points_exact.cuh", "points_fast.cuh", "bc_exact.cuh", "warmstart.h", "tile_engine.h",
+HEADERS = [os.path.join(ROOT, "include", "unet.h"), "acs_dev.cuh", "kernels.h", "fast.h", "engine.cuh", "engine_api.h", "chip_engine.h", "chip_engine.cuh", "chip_launch.inl", "points_exact.cuh", "points_fast.cuh", "bc_exact.cuh", "warmstart.h", "tile_engine.h",
            "../unet/csrc/gemm_tc.cuh"]
 
 

@@ -14,12 +14,14 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 
 #include "../../include/acs.h"
 #include "acs_dev.cuh"
 #include "fast.h"
+#include "chip_engine.h"
 #include "engine_api.h"
 #include "kernels.h"
 #include "tile_engine.h"
@@ -113,6 +115,10 @@ struct Batch {
   int staged = 1;        // FAST engine: stage stencil arrays in shared memory where they fit
   int last_staged = 0;   // the last engine launch used the staged kernel
   std::vector<int> cluster_override;  // per case: CTAs of its cluster (0 = from nodes_per_cta)
+  std::vector<char> chip_ok;          // per case: its constants suit the on-chip engine's arithmetic
+  bool user_nodes = false;            // nodes_per_cta was set by the caller
+  std::vector<int> chip_k;            // per case: CTAs of its on-chip cluster (0 = cluster engine); built on
+                                      // first use, emptied when a launch option changes
   int* d_cases = nullptr;
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> ev;
@@ -216,6 +222,18 @@ bool binary_porosity(const acs_grid& g, double* phi) {
   }
   *phi = ph < 0.0 ? 1.0 : ph;
   return true;
+}
+
+// Divisors of the EXACT on-chip arithmetic (chip_exact.cu): metric differences, porosity and drag
+// constants must be positive and far from the exponent limits.
+bool chip_divisors(const acs_grid& g, const acs_params& p, double phi) {
+  auto ok = [](double v) { return v >= 0x1p-60 && v <= 0x1p60; };
+  bool r = ok(phi) && ok(1.0 * (phi - 1.0) + 1.0) && ok(p.Re * p.Da) && ok(p.Re) && ok(p.Pe) && ok(p.Re * p.Sc);
+  for (int i = 1; i < g.imax; ++i) r = r && ok(g.x[i] - g.x[i - 1]);
+  for (int j = 1; j < g.jmax; ++j) r = r && ok(g.y[j] - g.y[j - 1]);
+  for (int i = 2; i < g.imax; ++i) r = r && ok(g.xm[i] - g.xm[i - 1]);  // interior cells only
+  for (int j = 2; j < g.jmax; ++j) r = r && ok(g.ym[j] - g.ym[j - 1]);
+  return r;
 }
 
 int push_ctl(Batch& b);
@@ -402,6 +420,7 @@ int create_batch(const acs_grid* grids_in, const acs_params* params, int n, Batc
   b->hc.resize(n);
   b->hk.assign(n, CaseCtl{});
   b->t_unity.assign(n, 0);
+  b->chip_ok.assign(n, 0);
   b->use_fast = fast;
   b->pool_bytes = head + total;
   cudaError_t e = cudaMalloc(&b->pool, b->pool_bytes);
@@ -476,6 +495,7 @@ int create_batch(const acs_grid* grids_in, const acs_params* params, int n, Batc
     double phi = 1.0;
     if (binary_porosity(g, &phi)) d.flags |= F_BINARY;
     d.phi = phi;
+    b->chip_ok[c] = (d.flags & F_BINARY) && pr.b_art == 0.0 && (fast || chip_divisors(g, pr, phi));
     if (pr.b_art != 0.0) d.flags |= F_BART;
     if (porous) d.flags |= F_POROUS;
     if (pr.InvFr2 != 0.0 && pr.solve_scalars) d.flags |= F_BUOY;
@@ -783,17 +803,86 @@ int cluster_size(const Batch& b, int c) {
   return K;
 }
 
-// One launch per cluster size, each on its own stream so the size classes run side by side.
+// Shared memory of one CTA when case c runs on chip in clusters of K (0: it does not fit, or the case
+// has more than one porosity, partly porous cells, artificial
+// divergence damping (b_art) or extreme constants).
+size_t chip_smem(const Batch& b, int c, int K, bool phys) {
+  const CaseDev& d = b.hc[c];
+  if (!b.chip_ok[c]) return 0;
+  const size_t s = sizeof(double) * (size_t)chip_layout(d.nx, d.ny, d.pitch, K, d.solve_scalars != 0, phys).total;
+  return s <= (size_t)CHIP_MAX_SMEM ? s : 0;
+}
+
+// CTAs of every case's on-chip cluster, 0 where the cluster engine takes the case.  A split that the
+// caller set (ACS_OPT_NODES_PER_CTA, acs_batch_set_cluster_size) is kept.  Otherwise the split with
+// the smallest modelled time of one pseudo-iteration of all cases: a case in K CTAs takes
+// CHIP_T0 + CHIP_T1 * (nodes of its largest strip), and the device runs as many clusters of K at once
+// as its GPCs hold (on a B200 15 of 9 CTAs, 11 of 10, 7 of 11 to 16).
+void chip_plan(Batch& b) {
+  if ((int)b.chip_k.size() == b.n) return;
+  b.chip_k.assign(b.n, 0);
+  std::vector<int> kmin(b.n, 0), kmax(b.n, 0), todo;
+  for (int c = 0; c < b.n; ++c) {
+    if (b.user_nodes || (c < (int)b.cluster_override.size() && b.cluster_override[c] > 0)) {
+      const int K = cluster_size(b, c);
+      if (chip_smem(b, c, K, false)) b.chip_k[c] = K;
+      continue;
+    }
+    kmax[c] = std::max(1, std::min(16, (b.hc[c].ny + 1) / 4));
+    for (int K = 1; K <= kmax[c] && !kmin[c]; ++K)
+      if (chip_smem(b, c, K, false)) kmin[c] = K;
+    if (kmin[c]) todo.push_back(c);
+  }
+  if (todo.empty()) return;
+  const double t0 = b.use_fast ? CHIP_T0_FAST : CHIP_T0_EXACT, t1 = b.use_fast ? CHIP_T1_FAST : CHIP_T1_EXACT;
+  double best = 0.0;
+  int best_k = 0;
+  for (int K = 1; K <= 16; ++K) {
+    int kk = 0;
+    std::vector<double> t;
+    for (int c : todo) {
+      const int k = std::min(std::max(K, kmin[c]), kmax[c]);
+      const CaseDev& d = b.hc[c];
+      kk = std::max(kk, k);
+      t.push_back((t0 + t1 * d.nx * ((d.ny + 1 + k - 1) / k)) * (d.solve_scalars ? 1.0 : 0.6));
+    }
+    const int slots = std::max(1, (b.use_fast ? chip_resident_fast : chip_resident_exact)(kk));
+    // longest first onto the slot that is free first
+    std::sort(t.begin(), t.end(), std::greater<double>());
+    std::vector<double> busy(std::min((size_t)slots, t.size()), 0.0);
+    for (double x : t) {
+      std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+      busy.back() += x;
+      std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+    }
+    const double end = *std::max_element(busy.begin(), busy.end());
+    if (!best_k || end < best) {
+      best = end;
+      best_k = K;
+    }
+  }
+  for (int c : todo) b.chip_k[c] = std::min(std::max(best_k, kmin[c]), kmax[c]);
+}
+
+// One launch per cluster size and engine, each on its own stream so the classes run side by side.
 int run_engine(Batch& b) {
-  std::vector<std::vector<int>> groups(17);
-  for (int c = 0; c < b.n; ++c) groups[cluster_size(b, c)].push_back(c);
+  chip_plan(b);
+  // classes 0..16: cluster engine by cluster size; from 17 on the on-chip engine by cluster size,
+  // with bit 0 of class / 17 - 1: the physical-step arrays on chip too, bit 1: QUICK
+  constexpr int kClasses = 5 * 17;
+  std::vector<std::vector<int>> groups(kClasses);
+  for (int c = 0; c < b.n; ++c) {
+    const int K = b.chip_k[c];
+    const int kind = 1 + (K && chip_smem(b, c, K, true) ? 1 : 0) + (b.hc[c].scheme == 0 ? 2 : 0);
+    groups[!K ? cluster_size(b, c) : 17 * kind + K].push_back(c);
+  }
   if (!b.d_cases) CU(cudaMalloc(&b.d_cases, sizeof(int) * b.n));
   std::vector<int> order;
-  std::vector<std::pair<int, int>> launches;  // (K, offset)
-  for (int K = 16; K >= 1; --K) {
-    if (groups[K].empty()) continue;
-    launches.push_back({K, (int)order.size()});
-    order.insert(order.end(), groups[K].begin(), groups[K].end());
+  std::vector<std::pair<int, int>> launches;  // (class, offset)
+  for (int k = kClasses - 1; k >= 0; --k) {
+    if (groups[k].empty()) continue;
+    launches.push_back({k, (int)order.size()});
+    order.insert(order.end(), groups[k].begin(), groups[k].end());
   }
   CU(cudaMemcpyAsync(b.d_cases, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, b.stream));
   for (int c = 0; c < b.n; ++c) {
@@ -814,11 +903,19 @@ int run_engine(Batch& b) {
   CU(cudaEventRecord(fork, b.stream));
   b.launches = 0;
   for (size_t g = 0; g < launches.size(); ++g) {
-    const int K = launches[g].first;
+    const int cls = launches[g].first, K = cls % 17;
     const int off = launches[g].second;
-    const int cnt = (int)groups[K].size();
+    const int cnt = (int)groups[cls].size();
     cudaStream_t s = g == 0 ? b.stream : b.side[g];
     if (g) CU(cudaStreamWaitEvent(s, fork, 0));
+    cudaError_t e;
+    if (cls >= 17) {
+      const bool phys = (cls / 17 - 1) & 1, quick = (cls / 17 - 1) & 2;
+      size_t smem = 0;
+      for (int q = 0; q < cnt; ++q) smem = std::max(smem, chip_smem(b, order[off + q], K, phys));
+      ChipArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err};
+      e = (b.use_fast ? launch_chip_fast : launch_chip_exact)(a, K, cnt, phys, quick, smem, s);
+    } else {
     // staging slot: the largest strip of the size class plus two halo rows on each side
     long long slot = 0;
     for (int q = 0; q < cnt; ++q) {
@@ -829,9 +926,10 @@ int run_engine(Batch& b) {
     const bool stg = b.use_fast && b.staged && b.ctas_per_sm == 1 &&
                      (long long)STAGE_SLOTS * slot * 8 <= kMaxStageBytes;
     EngineArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err, stg ? (int)slot : 0};
-    cudaError_t e = b.use_fast ? launch_engine_fast(a, K, cnt, s, b.l1_loads, b.threads, b.ctas_per_sm, stg ? 1 : 0)
-                               : launch_engine_exact(a, K, cnt, s);
+    e = b.use_fast ? launch_engine_fast(a, K, cnt, s, b.l1_loads, b.threads, b.ctas_per_sm, stg ? 1 : 0)
+                   : launch_engine_exact(a, K, cnt, s);
     b.last_staged = stg ? 1 : 0;
+    }
     if (e != cudaSuccess) {
       cudaEventDestroy(fork);
       return fail(ACS_E_CUDA, std::string("engine launch (cluster ") + std::to_string(K) + "): " + cudaGetErrorString(e));
@@ -1116,6 +1214,7 @@ int acs_batch_set_cluster_size(acs_batch* h, int c, int ctas) {
   if (ctas < 0 || ctas > 16) return acs::fail(ACS_E_ARG, "cluster size must be 0..16");
   if ((int)b.cluster_override.size() < b.n) b.cluster_override.assign(b.n, 0);
   b.cluster_override[c] = ctas;
+  b.chip_k.clear();
   return ACS_OK;
 }
 
@@ -1153,6 +1252,8 @@ int acs_batch_set_option(acs_batch* h, int option, long long value) {
     case ACS_OPT_NODES_PER_CTA:
       if (value < 64 || value > (1 << 22)) return acs::fail(ACS_E_ARG, "nodes per CTA out of range");
       b.nodes_per_cta = (int)value;
+      b.user_nodes = true;
+      b.chip_k.clear();
       return ACS_OK;
     case ACS_OPT_L1_LOADS:
       b.l1_loads = value ? 1 : 0;
