@@ -221,12 +221,15 @@ int acs_solve_u_static(const acs_params* p, const acs_grid* grid_dev, const doub
 /* Solver options (no reference counterpart). */
 enum acs_option {
   ACS_OPT_ENGINE = 1,        /* 0 (default): persistent cluster engine, one thread-block cluster
-                                per case runs whole physical steps in one launch;
+                                per case runs whole physical steps in one launch, on chip
+                                (state in the cluster's shared memory) where the case fits;
                                 1: CUDA graph of per-stage kernels with a device WHILE node;
                                 2: tile engine, ACS_ARITH_FAST only (ACS_E_UNSUPPORTED otherwise):
                                    32 x 32-node tiles of every active case loaded into shared
                                    memory by TMA, four stage kernels per pseudo-iteration in a CUDA graph
-                                   with a device WHILE node -- the fastest for many cases.  Setting
+                                   with a device WHILE node -- the fastest for many cases; a batch
+                                   whose cases all fit on chip and iterate faster there (a few
+                                   cases) runs as with 0.  Setting
                                    it builds the tile table and tensor maps (device memory).  With
                                    the environment variable ACS_NO_CONDITIONAL_GRAPH set, engines 1
                                    and 2 loop from the host instead (one graph launch per

@@ -119,6 +119,7 @@ struct Batch {
   bool user_nodes = false;            // nodes_per_cta was set by the caller
   std::vector<int> chip_k;            // per case: CTAs of its on-chip cluster (0 = cluster engine); built on
                                       // first use, emptied when a launch option changes
+  double chip_us = 0.0;               // modelled time of a pseudo-iteration of all cases on chip (0: not all fit)
   int* d_cases = nullptr;
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> ev;
@@ -695,6 +696,7 @@ int build_graph(Batch& b, int n_steps) {
 
 int run_engine(Batch& b);
 int run_graph(Batch& b, int n_steps);
+bool chip_beats_tiles(Batch& b);
 
 int run_batch(Batch& b, int n_steps, int* itc, int* iters, double* err, int* status) {
   if (n_steps <= 0) return fail(ACS_E_ARG, "n_steps must be positive");
@@ -728,7 +730,7 @@ int run_batch(Batch& b, int n_steps, int* itc, int* iters, double* err, int* sta
   r = push_ctl(b);
   if (r) return r;
   CU(cudaMemsetAsync(b.d_nactive, 0, 256, b.stream));
-  if (b.engine == 0) {
+  if (b.engine == 0 || (b.engine == 2 && chip_beats_tiles(b))) {
     r = run_engine(b);
     if (r) return r;
   } else {
@@ -821,6 +823,7 @@ size_t chip_smem(const Batch& b, int c, int K, bool phys) {
 void chip_plan(Batch& b) {
   if ((int)b.chip_k.size() == b.n) return;
   b.chip_k.assign(b.n, 0);
+  b.chip_us = 0.0;
   std::vector<int> kmin(b.n, 0), kmax(b.n, 0), todo;
   for (int c = 0; c < b.n; ++c) {
     if (b.user_nodes || (c < (int)b.cluster_override.size() && b.cluster_override[c] > 0)) {
@@ -862,6 +865,20 @@ void chip_plan(Batch& b) {
     }
   }
   for (int c : todo) b.chip_k[c] = std::min(std::max(best_k, kmin[c]), kmax[c]);
+  if ((int)todo.size() == b.n) b.chip_us = best;
+}
+
+// Whether a batch on the tile engine is faster on chip: the tile engine's seven launches of a
+// pseudo-iteration take at least 50 us, and 0.165 us per 1000 nodes once they fill the device (measured:
+// 45,000 nodes 51 us, 0.52 million 105, 1.5 million 273, 4.1 million 770), while a few cases in clusters
+// iterate side by side in 15 to 30 us (3 cases of 101 x 147: 51 us against 19).  Only a clear advantage
+// of the modelled times counts.
+bool chip_beats_tiles(Batch& b) {
+  if (getenv("ACS_NO_CONDITIONAL_GRAPH")) return false;  // a profiler wants the tile kernels
+  chip_plan(b);
+  double nodes = 0.0;
+  for (int c = 0; c < b.n; ++c) nodes += (double)b.hc[c].nx * b.hc[c].ny;
+  return b.chip_us > 0.0 && b.chip_us < 0.8 * std::max(50.0, 30.0 + 1.65e-4 * nodes);
 }
 
 // One launch per cluster size and engine, each on its own stream so the classes run side by side.

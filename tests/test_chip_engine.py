@@ -85,3 +85,16 @@ def test_cases_left_to_the_cluster_engine(gpu, orc):
     _compare(gpu, orc, prm, mesh, (0,), [(2, 1)])
     prm, mesh = _case(gpu, "full", 210, 205, itc_max=3)
     _compare(gpu, orc, prm, mesh, (0,), [(1, 1)])
+
+
+@pytest.mark.parametrize("nx,ny", [(61, 45), (70, 33), (20, 26)])
+def test_tile_kernels_on_small_cases(gpu, orc, monkeypatch, nx, ny):
+    """Small batches on the tile engine run on chip; with the host-polled loop they stay on the tile
+    kernels.  Both against the oracle at the FAST arithmetic's bound (1e-10)."""
+    from test_tile_engine import _tile_vs_oracle
+    item = gpu.configs.channel_case(nx, ny, seed=nx, Re=150.0, scheme=gpu.SCHEME_QUICK,
+                                    block=gpu.configs.centred_block(2, 1, 0.3), porosity=0.5, Da=1e-3, Cf=0.55, Ri=0.8,
+                                    scalars=True, itc_max=100)
+    _tile_vs_oracle(gpu, orc, [item], 2)
+    monkeypatch.setenv("ACS_NO_CONDITIONAL_GRAPH", "1")
+    _tile_vs_oracle(gpu, orc, [item], 2)
