@@ -22,6 +22,39 @@ using bf16 = __nv_bfloat16;
 constexpr int T = 256;
 inline unsigned blocks(long long n) { return (unsigned)((n + T - 1) / T < 65535LL * 64 ? (n + T - 1) / T : 65535LL * 64); }
 
+// Any C: one thread per 16-byte vector of 8 consecutive k of one pixel, whose up to 8 channels come from one
+// or two taps.  Index arithmetic in 32 bits, once per vector: the kernel that computed one element per
+// thread with 64-bit divisions took 1501 us for 64 canvases of 160 x 160 with 11 channels.
+__global__ void k_im2col_any(const bf16* __restrict__ X, int H, int W, int C, int Kp, unsigned n, uint4* __restrict__ col) {
+  const unsigned k8 = (unsigned)Kp >> 3;
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const unsigned m = q / k8;
+    int k = (int)(q - m * k8) * 8;
+    const int x = (int)(m % (unsigned)W), y = (int)(m / (unsigned)W % (unsigned)H);
+    int tap = k / C, c = k - tap * C;
+    unsigned short v[8];
+    const unsigned short* src = nullptr;
+    bool ok = false;
+    auto set_tap = [&]() {
+      const int ky = tap / 3, kx = tap - 3 * ky;
+      ok = tap < 9 && (unsigned)(y + ky - 1) < (unsigned)H && (unsigned)(x + kx - 1) < (unsigned)W;
+      src = reinterpret_cast<const unsigned short*>(X) + ((long long)m + (ky - 1) * W + kx - 1) * C;
+    };
+    set_tap();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = ok ? src[c] : (unsigned short)0;
+      if (++c == C) {
+        c = 0;
+        ++tap;
+        set_tap();
+      }
+    }
+    col[q] = make_uint4(v[0] | (unsigned)v[1] << 16, v[2] | (unsigned)v[3] << 16, v[4] | (unsigned)v[5] << 16,
+                        v[6] | (unsigned)v[7] << 16);
+  }
+}
+
 __global__ void k_im2col(const bf16* __restrict__ X, int B, int H, int W, int C, int Kp, bf16* __restrict__ col) {
   const long long n = (long long)B * H * W * Kp;
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
@@ -103,6 +136,42 @@ __global__ void k_pool_fwd(const bf16* __restrict__ X, int B, int H, int W, int 
     const float s = __bfloat162float(X[i0]) + __bfloat162float(X[i0 + C]) + __bfloat162float(X[i0 + (long long)W * C]) +
                     __bfloat162float(X[i0 + (long long)W * C + C]);
     Y[q] = __float2bfloat16_rn(0.25f * s);
+  }
+}
+
+// The forward movements below for C a multiple of 8 and aligned tensors: one thread per 16-byte vector
+// of 8 channels, 32-bit index arithmetic.
+__device__ __forceinline__ unsigned avg4(unsigned a, unsigned b, unsigned c, unsigned d) {
+  auto f = [](unsigned v) { return *reinterpret_cast<const __nv_bfloat162*>(&v); };
+  const float2 x = __bfloat1622float2(f(a)), y = __bfloat1622float2(f(b)), z = __bfloat1622float2(f(c)),
+               w = __bfloat1622float2(f(d));
+  const __nv_bfloat162 r = __floats2bfloat162_rn(0.25f * (x.x + y.x + z.x + w.x), 0.25f * (x.y + y.y + z.y + w.y));
+  return *reinterpret_cast<const unsigned*>(&r);
+}
+__global__ void k_pool_fwd_v8(const uint4* __restrict__ X, int h, int w, int C8, unsigned n, uint4* __restrict__ Y) {
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const unsigned p = q / (unsigned)C8, c = q - p * C8, x = p % (unsigned)w, by = p / (unsigned)w;  // by = b*h + y
+    const uint4* s = X + ((long long)by * 2 * (2 * w) + 2 * x) * C8 + c;
+    const uint4 a = s[0], b = s[C8], e = s[(long long)2 * w * C8], f = s[(long long)(2 * w + 1) * C8];
+    Y[q] = make_uint4(avg4(a.x, b.x, e.x, f.x), avg4(a.y, b.y, e.y, f.y), avg4(a.z, b.z, e.z, f.z), avg4(a.w, b.w, e.w, f.w));
+  }
+}
+// one thread per coarse vector: one load, four stores
+__global__ void k_up_fwd_v8(const uint4* __restrict__ X, int w, int C8, unsigned n, uint4* __restrict__ Y, int ld8, int c08) {
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const unsigned p = q / (unsigned)C8, c = q - p * C8, x = p % (unsigned)w, by = p / (unsigned)w;
+    const uint4 v = X[q];
+    uint4* d = Y + ((long long)by * 2 * (2 * w) + 2 * x) * ld8 + c08 + c;
+    d[0] = v;
+    d[ld8] = v;
+    d[(long long)2 * w * ld8] = v;
+    d[(long long)(2 * w + 1) * ld8] = v;
+  }
+}
+__global__ void k_copy_ch_v8(const uint4* __restrict__ X, int C8, unsigned n, uint4* __restrict__ Y, int ld8, int c08) {
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const unsigned p = q / (unsigned)C8, c = q - p * C8;
+    Y[(long long)p * ld8 + c08 + c] = X[q];
   }
 }
 
@@ -274,6 +343,11 @@ __global__ void k_normalize(const float* X, long long M, int C, const float* __r
   }
 }
 
+// Whether tensors with these channel counts and base addresses can be moved as 16-byte vectors, n of
+// them, with 32-bit indices.
+inline bool vec8(long long n, int c0, int c1, int c2, const void* a, const void* b) {
+  return ((c0 | c1 | c2) & 7) == 0 && n < (1ll << 31) && !((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15);
+}
 inline int ret(cudaStream_t) { return cudaGetLastError() == cudaSuccess ? 0 : 3; }
 
 }  // namespace
@@ -288,6 +362,11 @@ int unet_im2col(const void* X, int B, int H, int W, int C, int Kp, void* col, vo
   if (!X || !col || Kp < 9 * C || (Kp & 7)) return 1;
   if ((C & 7) == 0 && Kp == 9 * C && !(reinterpret_cast<uintptr_t>(X) & 15) && !(reinterpret_cast<uintptr_t>(col) & 15)) {
     k_im2col_v8<<<blocks((long long)B * H * W * 9 * (C >> 3)), T, 0, S_>>>((const uint4*)X, B, H, W, C, (uint4*)col);
+    return ret(S_);
+  }
+  const long long nv = (long long)B * H * W * (Kp >> 3);
+  if (nv < (1ll << 31) && !(reinterpret_cast<uintptr_t>(col) & 15)) {
+    k_im2col_any<<<blocks(nv), T, 0, S_>>>((const bf16*)X, H, W, C, Kp, (unsigned)nv, (uint4*)col);
     return ret(S_);
   }
   k_im2col<<<blocks((long long)B * H * W * Kp), T, 0, S_>>>((const bf16*)X, B, H, W, C, Kp, (bf16*)col);
@@ -306,6 +385,11 @@ int unet_transpose_bf16(const void* src, int rows, int cols, int lds, void* dst,
 }
 int unet_pool_fwd(const void* X, int B, int H, int W, int C, void* Y, void* stream) {
   if (!X || !Y || (H & 1) || (W & 1)) return 1;
+  const long long nv = (long long)B * (H / 2) * (W / 2) * (C >> 3);
+  if (vec8(4 * nv, C, 0, 0, X, Y)) {
+    k_pool_fwd_v8<<<blocks(nv), T, 0, S_>>>((const uint4*)X, H / 2, W / 2, C >> 3, (unsigned)nv, (uint4*)Y);
+    return ret(S_);
+  }
   k_pool_fwd<<<blocks((long long)B * H * W * C / 4), T, 0, S_>>>((const bf16*)X, B, H, W, C, (bf16*)Y);
   return ret(S_);
 }
@@ -316,6 +400,11 @@ int unet_pool_bwd(const float* dY, int B, int H, int W, int C, float* dX, int ac
 }
 int unet_up_fwd(const void* X, int B, int h, int w, int C, void* Y, int ldy, int cofs, void* stream) {
   if (!X || !Y || cofs + C > ldy) return 1;
+  const long long nv = (long long)B * h * w * (C >> 3);
+  if (vec8(nv, C, ldy, cofs, X, Y)) {
+    k_up_fwd_v8<<<blocks(nv), T, 0, S_>>>((const uint4*)X, w, C >> 3, (unsigned)nv, (uint4*)Y, ldy >> 3, cofs >> 3);
+    return ret(S_);
+  }
   k_up_fwd<<<blocks((long long)B * 4 * h * w * C), T, 0, S_>>>((const bf16*)X, B, h, w, C, (bf16*)Y, ldy, cofs);
   return ret(S_);
 }
@@ -326,6 +415,11 @@ int unet_up_bwd(const float* dY, int ldy, int cofs, int B, int h, int w, int C, 
 }
 int unet_copy_channels(const void* X, long long M, int C, void* Y, int ldy, int cofs, void* stream) {
   if (!X || !Y || cofs + C > ldy) return 1;
+  const long long nv = M * (C >> 3);
+  if (vec8(nv, C, ldy, cofs, X, Y)) {
+    k_copy_ch_v8<<<blocks(nv), T, 0, S_>>>((const uint4*)X, C >> 3, (unsigned)nv, (uint4*)Y, ldy >> 3, cofs >> 3);
+    return ret(S_);
+  }
   k_copy_ch<<<blocks(M * C), T, 0, S_>>>((const bf16*)X, M, C, (bf16*)Y, ldy, cofs);
   return ret(S_);
 }
