@@ -27,6 +27,13 @@ int unet_gemm(const void* A, int lda, const void* B, int ldb, int M, int N, int 
 int unet_conv3x3(const void* X, int B, int H, int W, int C, const void* Wt, int ldw, int Cout, int epilogue,
                  float* Cf, void* Y, int ldc, const float* bias, int relu, int* err, void* stream);
 
+/* The same convolution for any channel count with a small window (the network's 11-channel input):
+ * Y = bf16(act(col(X) Wt^T + bias)), col and Kp = 9C rounded up to 8 as for unet_im2col, ldw >= Kp,
+ * Cout <= 64.  Returns 1 where the window does not fit in shared memory.  Same results as
+ * unet_im2col + unet_gemm. */
+int unet_conv3x3_gather(const void* X, int B, int H, int W, int C, const void* Wt, int ldw, int Kp, int Cout,
+                        void* Y, int ldc, const float* bias, int relu, int* err, void* stream);
+
 /* Layer kernels.  Activations are NHWC ([pixels][channels], pixels ordered batch, row, column).
  * A 3x3 "same" convolution is the GEMM col(X) W^T with col(X)[m][(ky*3+kx)*C + c] =
  * X[b][y+ky-1][x+kx-1][c] (zero outside the canvas and for k >= 9C; Kp = padded K, multiple of 8). */

@@ -30,6 +30,7 @@ I = C.c_int
 _SIG = {
     "unet_gemm": [V, I, V, I, I, I, I, I, V, V, I, V, I, I, V, V],
     "unet_conv3x3": [V, I, I, I, I, V, I, I, I, V, V, I, V, I, V, V],
+    "unet_conv3x3_gather": [V, I, I, I, I, V, I, I, I, V, I, V, I, V, V],
     "unet_im2col": [V, I, I, I, I, I, V, V],
     "unet_col2im": [V, I, I, I, I, I, V, V],
     "unet_transpose_bf16": [V, I, I, I, V, I, V],
@@ -263,6 +264,11 @@ class UNet:
                 code = K.unet_conv3x3(_p(X), B, H, W, L.cin, wb, L.kp, L.cout, 2, None, _p(Y), L.cout, bias,
                                       1 if L.relu else 0, _p(self.err), s)
             _ok(code, f"conv3x3 {L.name}")
+            return
+        if self.implicit and not out_f32 and L.cout <= 64 and L.cin < 16:
+            # steps of 16 cross taps: the CTA gathers col's rows from its window
+            _ok(K.unet_conv3x3_gather(_p(X), B, H, W, L.cin, wb, L.kp, L.kp, L.cout, _p(Y), L.cout, bias,
+                                      1 if L.relu else 0, _p(self.err), s), f"conv3x3 {L.name}")
             return
         col = ws["col"]
         _ok(K.unet_im2col(_p(X), B, H, W, L.cin, L.kp, _p(col), s), "im2col")
