@@ -34,6 +34,16 @@ int unet_conv3x3(const void* X, int B, int H, int W, int C, const void* Wt, int 
 int unet_conv3x3_gather(const void* X, int B, int H, int W, int C, const void* Wt, int ldw, int Kp, int Cout,
                         void* Y, int ldc, const float* bias, int relu, int* err, void* stream);
 
+/* Gradients of the 3x3 convolution Y = col(X) W^T with W^T [9C][Cout] (row tap*C + c):
+ * gW[9C][Cout] += col(X)^T dZ (FP32 atomics), dX[pixel][C] = col2im(dZ W), same values as the GEMM and
+ * unet_col2im.  Cout a multiple of 8; dZ, Wt, gW, dX (and X where C is a multiple of 8) 16-byte aligned.
+ * unet_conv3x3_dx_fits tells whether dX's window fits in shared memory (else unet_conv3x3_dx returns 1). */
+int unet_conv3x3_dw(const void* X, const void* dZ, int B, int H, int W, int C, int Cout, float* gW, int* err,
+                    void* stream);
+int unet_conv3x3_dx_fits(int C, int Cout);
+int unet_conv3x3_dx(const void* dZ, const void* Wt, int B, int H, int W, int C, int Cout, float* dX, int* err,
+                    void* stream);
+
 /* Layer kernels.  Activations are NHWC ([pixels][channels], pixels ordered batch, row, column).
  * A 3x3 "same" convolution is the GEMM col(X) W^T with col(X)[m][(ky*3+kx)*C + c] =
  * X[b][y+ky-1][x+kx-1][c] (zero outside the canvas and for k >= 9C; Kp = padded K, multiple of 8). */
@@ -55,6 +65,9 @@ int unet_take_channels(const float* dY, int ldy, int cofs, long long M, int C, f
                        void* stream);
 /* dZ = bf16(relu ? dY * [Y > 0] : dY) over n values */
 int unet_act_bwd(const float* dY, const void* Y, long long n, int relu, void* dZ, void* stream);
+/* unet_act_bwd over [M][C] and db[c] += sum_m dZ[m][c] in one pass (C a multiple of 8 up to 1024, tensors
+ * 16-byte aligned) */
+int unet_act_bias_bwd(const float* dY, const void* Y, long long M, int C, int relu, void* dZ, float* db, void* stream);
 /* db[c] += sum_m dZ[m][c] (db must be zeroed by the caller) */
 int unet_bias_grad(const void* dZ, long long M, int C, float* db, void* stream);
 int unet_f32_to_bf16(const float* a, long long n, void* b, void* stream);

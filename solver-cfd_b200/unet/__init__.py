@@ -3,8 +3,8 @@
 Every product is the tcgen05 GEMM of ``unet_gemm``: a 3x3 "same" convolution is
 ``col(X) @ W^T`` with ``col`` built by ``unet_im2col`` (NHWC activations, K index
 ``(ky*3+kx)*Cin + c`` padded to a multiple of 8); in the forward pass, layers whose Cin is a
-multiple of 8 use ``unet_conv3x3``, the same GEMM gathering ``col`` on the fly.  Its gradients are ``dW^T = col(X)^T dZ``
-(split-K GEMM with FP32 atomics) and ``dX = col2im(dZ W)``.  Pooling (2x2 average), nearest
+multiple of 8 use ``unet_conv3x3``, the same product without ``col`` in memory.  Its gradients are ``dW^T = col(X)^T dZ``
+(``unet_conv3x3_dw``) and ``dX = col2im(dZ W)`` (``unet_conv3x3_dx``), neither with a matrix of col's size.  Pooling (2x2 average), nearest
 upsampling, skip concatenation, ReLU backward, bias gradients, the masked MSE and Adam are the
 kernels of ``unet_ops.cu``.  torch only allocates device memory and orders work on its current
 stream; it performs none of the network's arithmetic.
@@ -31,6 +31,10 @@ _SIG = {
     "unet_gemm": [V, I, V, I, I, I, I, I, V, V, I, V, I, I, V, V],
     "unet_conv3x3": [V, I, I, I, I, V, I, I, I, V, V, I, V, I, V, V],
     "unet_conv3x3_gather": [V, I, I, I, I, V, I, I, I, V, I, V, I, V, V],
+    "unet_conv3x3_dw": [V, V, I, I, I, I, I, V, V, V],
+    "unet_conv3x3_dx_fits": [I, I],
+    "unet_conv3x3_dx": [V, V, I, I, I, I, I, V, V, V],
+    "unet_act_bias_bwd": [V, V, LL, I, I, V, V, V],
     "unet_im2col": [V, I, I, I, I, I, V, V],
     "unet_col2im": [V, I, I, I, I, I, V, V],
     "unet_transpose_bf16": [V, I, I, I, V, I, V],
@@ -232,16 +236,18 @@ class UNet:
         ws["x"] = torch.zeros(Ms[0] * self.cin, **bf)
         ws["y"] = torch.zeros(Ms[0] * OUT_PAD, **f32)
         ws["dy"] = torch.zeros(Ms[0] * OUT_PAD, **f32)
-        max_col = max(Ms[self._level(L)] * L.kp for L in self.convs)
         max_z = max(Ms[self._level(L)] * L.cout for L in self.convs)
-        ws["col"] = torch.zeros(max_col, **bf)
-        ws["colT"] = torch.zeros(max_col, **bf)
-        ws["dcol"] = torch.zeros(max_col, **f32)
         ws["dz"] = torch.zeros(max_z, **bf)
-        ws["dzT"] = torch.zeros(max_z, **bf)
         ws["loss"] = torch.zeros(1, **f32)
         self._ws[key] = ws
         return ws
+
+    def _scratch(self, ws, name, n, dtype):
+        """A buffer of at least n values for the layers whose sizes need col or dcol in memory, kept with
+        the workspace."""
+        if name not in ws or ws[name].numel() < n:
+            ws[name] = self.torch.empty(n, dtype=dtype, device=self.dev)
+        return ws[name]
 
     @staticmethod
     def _level(L):
@@ -270,7 +276,7 @@ class UNet:
             _ok(K.unet_conv3x3_gather(_p(X), B, H, W, L.cin, wb, L.kp, L.kp, L.cout, _p(Y), L.cout, bias,
                                       1 if L.relu else 0, _p(self.err), s), f"conv3x3 {L.name}")
             return
-        col = ws["col"]
+        col = self._scratch(ws, "col", M * L.kp, self.torch.bfloat16)
         _ok(K.unet_im2col(_p(X), B, H, W, L.cin, L.kp, _p(col), s), "im2col")
         if out_f32:
             code = K.unet_gemm(_p(col), L.kp, wb, L.kp, M, L.cout, L.kp, 3, _p(Y), None, L.cout, bias, 0, 1,
@@ -320,22 +326,23 @@ class UNet:
         s = self._stream()
         B, H, W = ws["B"], ws["H"] >> lvl, ws["W"] >> lvl
         M = B * H * W
-        dz, dzT, col, colT, dcol = ws["dz"], ws["dzT"], ws["col"], ws["colT"], ws["dcol"]
-        _ok(K.unet_act_bwd(_p(dY), _p(Yact) if L.relu else None, M * L.cout, 1 if L.relu else 0, _p(dz), s),
-            "act_bwd")
+        dz = ws["dz"]
         gb = self.grad.data_ptr() + 4 * L.off_b
-        _ok(K.unet_bias_grad(_p(dz), M, L.cout, gb, s), "bias_grad")
-        _ok(K.unet_transpose_bf16(_p(dz), M, L.cout, L.cout, _p(dzT), M, s), "transpose dz")
-        _ok(K.unet_im2col(_p(X), B, H, W, L.cin, L.kp, _p(col), s), "im2col")
-        _ok(K.unet_transpose_bf16(_p(col), M, L.kp, L.kp, _p(colT), M, s), "transpose col")
+        if L.cout <= 1024:
+            _ok(K.unet_act_bias_bwd(_p(dY), _p(Yact) if L.relu else None, M, L.cout, 1 if L.relu else 0, _p(dz), gb, s),
+                "act_bias_bwd")
+        else:
+            _ok(K.unet_act_bwd(_p(dY), _p(Yact) if L.relu else None, M * L.cout, 1 if L.relu else 0, _p(dz), s), "act_bwd")
+            _ok(K.unet_bias_grad(_p(dz), M, L.cout, gb, s), "bias_grad")
         gw = self.grad.data_ptr() + 4 * L.off_w
-        tiles = ((L.kp + 127) // 128) * max(1, (L.cout + 255) // 256)
-        ktiles = (M + 63) // 64
-        splits = max(1, min(ktiles, (4 * 148 + tiles - 1) // tiles))
-        _ok(K.unet_gemm(_p(colT), M, _p(dzT), M, L.kp, L.cout, M, 1, gw, None, L.cout, None, 0, splits,
-                        _p(self.err), s), f"gemm dW {L.name}")
-        if dX is not None:
-            wt = self.wt_bf16.data_ptr() + 2 * L.off_w
+        _ok(K.unet_conv3x3_dw(_p(X), _p(dz), B, H, W, L.cin, L.cout, gw, _p(self.err), s), f"dW {L.name}")
+        if dX is None:
+            return
+        wt = self.wt_bf16.data_ptr() + 2 * L.off_w
+        if K.unet_conv3x3_dx_fits(L.cin, L.cout):
+            _ok(K.unet_conv3x3_dx(_p(dz), wt, B, H, W, L.cin, L.cout, _p(dX), _p(self.err), s), f"dX {L.name}")
+        else:
+            dcol = self._scratch(ws, "dcol", M * L.kp, self.torch.float32)
             _ok(K.unet_gemm(_p(dz), L.cout, wt, L.cout, M, L.kp, L.cout, 0, _p(dcol), None, L.kp, None, 0, 1,
                             _p(self.err), s), f"gemm dX {L.name}")
             _ok(K.unet_col2im(_p(dcol), B, H, W, L.cin, L.kp, _p(dX), s), "col2im")

@@ -3,6 +3,7 @@
 #include <cudaTypedefs.h>
 
 #include "../../../include/unet.h"
+#include "conv_grad_tc.cuh"
 #include "conv_tc.cuh"
 #include "gemm_tc.cuh"
 
@@ -102,6 +103,34 @@ cudaError_t conv_bn(const ConvCall& c, int bn) {
   }
 }
 
+template <int BN>
+cudaError_t dw_go(DwArgs a, cudaStream_t s) {
+  const int smem = 2 * dw_stage<BN>();
+  auto k = k_conv_dw<BN>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  a.nco = (a.N + BN - 1) / BN;
+  k<<<dim3((unsigned)((a.tiles + DW_TILES - 1) / DW_TILES), (unsigned)(3 * a.nco * ((a.C + 127) / 128))), TC_THREADS, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+int dx_smem(int N, int bn) {
+  const int kpad = (N + 15) / 16 * 16;
+  return (kpad >> 3) * cv_plane(1) + DX_RING * bn * kpad * 2;
+}
+// Input channels of a CTA: all of them up to 96, else blocks of 64.
+int dx_bn(int C) { return C <= 32 ? 32 : C <= 64 ? 64 : C <= 96 ? 96 : 64; }
+
+template <int BN>
+cudaError_t dx_go(const DxArgs& a, int batch, cudaStream_t s) {
+  const int smem = dx_smem(a.N, BN);
+  auto k = k_conv_dx<BN>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  k<<<dim3((unsigned)(batch * a.ty * a.tx), (unsigned)((a.C + BN - 1) / BN)), TC_THREADS, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
 ConvArgs conv_args(const void* X, int H, int W, int C, int K, int Cout, float* Cf, void* Y, int ldc, const float* bias,
                    int relu, int* err) {
   ConvArgs c{};
@@ -198,5 +227,55 @@ extern "C" int unet_conv3x3_gather(const void* X, int B, int H, int W, int C, co
   if (gather_smem(C, Kp, bn) > kConvSmem) return 1;
   ConvCall c{conv_args(X, H, W, C, Kp, Cout, nullptr, Y, ldc, bias, relu, err), Wt, ldw, B, static_cast<cudaStream_t>(stream)};
   const cudaError_t e = bn == 32 ? conv_go<32, 1, EPI_BIAS_BF16, true>(c) : conv_go<64, 1, EPI_BIAS_BF16, true>(c);
+  return e == cudaSuccess ? 0 : 3;
+}
+
+extern "C" int unet_conv3x3_dw(const void* X, const void* dZ, int B, int H, int W, int C, int Cout, float* gW, int* err,
+                               void* stream) {
+  using namespace unet;
+  if (!X || !dZ || !gW || B <= 0 || H <= 0 || W <= 0 || C <= 0 || Cout <= 0 || (Cout & 7) ||
+      (long long)B * H * W > 0x7fffffffLL)
+    return 1;
+  if ((reinterpret_cast<uintptr_t>(dZ) & 15) || (reinterpret_cast<uintptr_t>(gW) & 15) ||
+      ((C & 7) == 0 && (reinterpret_cast<uintptr_t>(X) & 15)))
+    return 1;
+  DwArgs a{};
+  a.X = static_cast<const __nv_bfloat16*>(X);
+  a.dZ = static_cast<const __nv_bfloat16*>(dZ);
+  a.batch = B; a.H = H; a.W = W; a.C = C; a.N = Cout;
+  a.tx = (W + CV_W - 1) / CV_W;
+  a.ty = (H + CV_H - 1) / CV_H;
+  a.tiles = B * a.tx * a.ty;
+  a.gW = gW;
+  a.err = err;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = Cout <= 16 ? dw_go<16>(a, s) : Cout <= 32 ? dw_go<32>(a, s) : Cout <= 64 ? dw_go<64>(a, s) : dw_go<128>(a, s);
+  return e == cudaSuccess ? 0 : 3;
+}
+
+extern "C" int unet_conv3x3_dx_fits(int C, int Cout) {
+  return C > 0 && Cout > 0 && (Cout & 7) == 0 && unet::dx_smem(Cout, unet::dx_bn(C)) <= unet::kConvSmem;
+}
+
+extern "C" int unet_conv3x3_dx(const void* dZ, const void* Wt, int B, int H, int W, int C, int Cout, float* dX, int* err,
+                               void* stream) {
+  using namespace unet;
+  if (!dZ || !Wt || !dX || B <= 0 || H <= 0 || W <= 0 || !unet_conv3x3_dx_fits(C, Cout) || (long long)B * H * W > 0x7fffffffLL)
+    return 1;
+  if ((reinterpret_cast<uintptr_t>(dZ) & 15) || (reinterpret_cast<uintptr_t>(Wt) & 15) || (reinterpret_cast<uintptr_t>(dX) & 15))
+    return 1;
+  DxArgs a{};
+  a.dZ = static_cast<const __nv_bfloat16*>(dZ);
+  a.Wt = static_cast<const __nv_bfloat16*>(Wt);
+  a.H = H; a.W = W; a.C = C; a.N = Cout;
+  a.tx = (W + CV_W - 1) / CV_W;
+  a.ty = (H + CV_H - 1) / CV_H;
+  a.plane = cv_plane(1);
+  a.kpad = (Cout + 15) / 16 * 16;
+  a.dX = dX;
+  a.err = err;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int bn = dx_bn(C);
+  const cudaError_t e = bn == 32 ? dx_go<32>(a, B, s) : bn == 96 ? dx_go<96>(a, B, s) : dx_go<64>(a, B, s);
   return e == cudaSuccess ? 0 : 3;
 }

@@ -238,6 +238,83 @@ __global__ void k_act_bwd(const float* __restrict__ dY, const bf16* __restrict__
   }
 }
 
+// Both at once: a thread keeps its 8 channels over its rows (active threads: whole groups of C / 8), so the
+// column sums stay in registers until the end.  The two kernels took 431 + 453 us for the gradients of 16
+// canvases of 160 x 160.
+__global__ void __launch_bounds__(T) k_act_bias_bwd(const float4* __restrict__ dY, const uint4* __restrict__ Y, unsigned M,
+                                                    int C8, int relu, uint4* __restrict__ dZ, float* __restrict__ db) {
+  extern __shared__ float sum[];  // [C]
+  for (int c = threadIdx.x; c < 8 * C8; c += blockDim.x) sum[c] = 0.f;
+  __syncthreads();
+  const int rows = blockDim.x / C8, c = threadIdx.x % C8, r = threadIdx.x / C8;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (r < rows) {
+    for (unsigned m = blockIdx.x * rows + r; m < M; m += gridDim.x * rows) {
+      const long long q = (long long)m * C8 + c;
+      const float4 a = __ldg(dY + 2 * q), b = __ldg(dY + 2 * q + 1);
+      float g[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      if (relu) {
+        const uint4 y = __ldg(Y + q);
+        const unsigned yw[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&yw[j]));
+          if (!(f.x > 0.f)) g[2 * j] = 0.f;
+          if (!(f.y > 0.f)) g[2 * j + 1] = 0.f;
+        }
+      }
+      unsigned zw[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(g[2 * j], g[2 * j + 1]);
+        zw[j] = *reinterpret_cast<const unsigned*>(&h);
+        const float2 f = __bfloat1622float2(h);
+        acc[2 * j] += f.x;
+        acc[2 * j + 1] += f.y;
+      }
+      dZ[q] = make_uint4(zw[0], zw[1], zw[2], zw[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) atomicAdd(&sum[8 * c + j], acc[j]);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < 8 * C8; k += blockDim.x) atomicAdd(db + k, sum[k]);
+}
+
+// The backward movements below for C a multiple of 4 and aligned tensors: one thread per four channels.
+__global__ void k_pool_bwd_v4(const float4* __restrict__ dY, int H, int W, int C4, unsigned n, float4* __restrict__ dX, int acc) {
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const unsigned p = q / (unsigned)C4, c = q - p * C4, x = p % (unsigned)W, by = p / (unsigned)W;
+    const unsigned b = by / (unsigned)H, y = by - b * H;
+    const float4 g = dY[((long long)(b * (H / 2) + y / 2) * (W / 2) + x / 2) * C4 + c];
+    float4 d = make_float4(0.25f * g.x, 0.25f * g.y, 0.25f * g.z, 0.25f * g.w);
+    if (acc) {
+      const float4 o = dX[q];
+      d = make_float4(o.x + d.x, o.y + d.y, o.z + d.z, o.w + d.w);
+    }
+    dX[q] = d;
+  }
+}
+__global__ void k_up_bwd_v4(const float4* __restrict__ dY, int ld4, int c04, int w, int C4, unsigned n, float4* __restrict__ dX) {
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const unsigned p = q / (unsigned)C4, c = q - p * C4, x = p % (unsigned)w, by = p / (unsigned)w;
+    const float4* s = dY + ((long long)by * 2 * (2 * w) + 2 * x) * ld4 + c04 + c;
+    const float4 a = s[0], b = s[ld4], e = s[(long long)2 * w * ld4], f = s[(long long)(2 * w + 1) * ld4];
+    dX[q] = make_float4(a.x + b.x + e.x + f.x, a.y + b.y + e.y + f.y, a.z + b.z + e.z + f.z, a.w + b.w + e.w + f.w);
+  }
+}
+__global__ void k_take_ch_v4(const float4* __restrict__ dY, int ld4, int c04, int C4, unsigned n, float4* __restrict__ dX, int acc) {
+  for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const unsigned p = q / (unsigned)C4, c = q - p * C4;
+    float4 g = dY[(long long)p * ld4 + c04 + c];
+    if (acc) {
+      const float4 o = dX[q];
+      g = make_float4(o.x + g.x, o.y + g.y, o.z + g.z, o.w + g.w);
+    }
+    dX[q] = g;
+  }
+}
+
 // db[c] += sum_m dZ[m][c]
 __global__ void k_colsum(const bf16* __restrict__ dZ, long long M, int C, float* __restrict__ db) {
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
@@ -348,6 +425,9 @@ __global__ void k_normalize(const float* X, long long M, int C, const float* __r
 inline bool vec8(long long n, int c0, int c1, int c2, const void* a, const void* b) {
   return ((c0 | c1 | c2) & 7) == 0 && n < (1ll << 31) && !((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15);
 }
+inline bool vec4(long long n, int c0, int c1, int c2, const void* a, const void* b) {
+  return ((c0 | c1 | c2) & 3) == 0 && n < (1ll << 31) && !((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15);
+}
 inline int ret(cudaStream_t) { return cudaGetLastError() == cudaSuccess ? 0 : 3; }
 
 }  // namespace
@@ -395,6 +475,11 @@ int unet_pool_fwd(const void* X, int B, int H, int W, int C, void* Y, void* stre
 }
 int unet_pool_bwd(const float* dY, int B, int H, int W, int C, float* dX, int accumulate, void* stream) {
   if (!dY || !dX || (H & 1) || (W & 1)) return 1;
+  const long long nv = (long long)B * H * W * (C >> 2);
+  if (vec4(nv, C, 0, 0, dY, dX)) {
+    k_pool_bwd_v4<<<blocks(nv), T, 0, S_>>>((const float4*)dY, H, W, C >> 2, (unsigned)nv, (float4*)dX, accumulate);
+    return ret(S_);
+  }
   k_pool_bwd<<<blocks((long long)B * H * W * C), T, 0, S_>>>(dY, B, H, W, C, dX, accumulate);
   return ret(S_);
 }
@@ -410,6 +495,11 @@ int unet_up_fwd(const void* X, int B, int h, int w, int C, void* Y, int ldy, int
 }
 int unet_up_bwd(const float* dY, int ldy, int cofs, int B, int h, int w, int C, float* dX, void* stream) {
   if (!dY || !dX || cofs + C > ldy) return 1;
+  const long long nv = (long long)B * h * w * (C >> 2);
+  if (vec4(nv, C, ldy, cofs, dY, dX)) {
+    k_up_bwd_v4<<<blocks(nv), T, 0, S_>>>((const float4*)dY, ldy >> 2, cofs >> 2, w, C >> 2, (unsigned)nv, (float4*)dX);
+    return ret(S_);
+  }
   k_up_bwd<<<blocks((long long)B * h * w * C), T, 0, S_>>>(dY, ldy, cofs, B, h, w, C, dX);
   return ret(S_);
 }
@@ -425,12 +515,26 @@ int unet_copy_channels(const void* X, long long M, int C, void* Y, int ldy, int 
 }
 int unet_take_channels(const float* dY, int ldy, int cofs, long long M, int C, float* dX, int accumulate, void* stream) {
   if (!dY || !dX || cofs + C > ldy) return 1;
+  const long long nv = M * (C >> 2);
+  if (vec4(nv, C, ldy, cofs, dY, dX)) {
+    k_take_ch_v4<<<blocks(nv), T, 0, S_>>>((const float4*)dY, ldy >> 2, cofs >> 2, C >> 2, (unsigned)nv, (float4*)dX, accumulate);
+    return ret(S_);
+  }
   k_take_ch<<<blocks(M * C), T, 0, S_>>>(dY, ldy, cofs, M, C, dX, accumulate);
   return ret(S_);
 }
 int unet_act_bwd(const float* dY, const void* Y, long long n, int relu, void* dZ, void* stream) {
   if (!dY || !dZ || (relu && !Y)) return 1;
   k_act_bwd<<<blocks(n), T, 0, S_>>>(dY, (const bf16*)Y, n, relu, (bf16*)dZ);
+  return ret(S_);
+}
+int unet_act_bias_bwd(const float* dY, const void* Y, long long M, int C, int relu, void* dZ, float* db, void* stream) {
+  if (!dY || !dZ || !db || (relu && !Y) || M <= 0 || M >= (1ll << 31) || C <= 0 || (C & 7) || C > 8 * T / 2) return 1;
+  if ((reinterpret_cast<uintptr_t>(dY) | reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(dZ)) & 15) return 1;
+  const int rows = T / (C >> 3);
+  const long long want = (M + rows - 1) / rows;
+  k_act_bias_bwd<<<(unsigned)(want < 148 * 8 ? want : 148 * 8), T, C * sizeof(float), S_>>>(
+      (const float4*)dY, (const uint4*)Y, (unsigned)M, C >> 3, relu, (uint4*)dZ, db);
   return ret(S_);
 }
 int unet_bias_grad(const void* dZ, long long M, int C, float* db, void* stream) {
