@@ -177,6 +177,9 @@ int acs_batch_destroy(acs_batch* b);
 int acs_batch_set_stream(acs_batch* b, void* cuda_stream);
 int acs_batch_set_field(acs_batch* b, int case_id, int field, const double* host);
 int acs_batch_get_field(acs_batch* b, int case_id, int field, double* host);
+/* n (1..14) distinct fields of a case at once: fields[q] from / to host[q]; the download waits once. */
+int acs_batch_set_fields(acs_batch* b, int case_id, int n, const int* fields, const double* const* host);
+int acs_batch_get_fields(acs_batch* b, int case_id, int n, const int* fields, double* const* host);
 /* comp_mean (comp_mean.f90:1-25) of case case_id's physical-step velocities computed on the device:
  * u(i,j) = (um(i+1,j) + um(i,j))/2, v(i,j) = (vm(i,j+1) + vm(i,j))/2 and sqrt(u^2 + v^2), the
  * velocity magnitude of the ParaView output (transient.f90:69-74); host arrays imax x jmax,

@@ -42,6 +42,7 @@ EXPORTED = (
     "acs_set_stream", "acs_solve_u", "acs_solve_v", "acs_solve_p", "acs_solve_z", "acs_solve_c",
     "acs_set_field", "acs_get_field", "acs_physical_steps", "acs_batch_create",
     "acs_batch_destroy", "acs_batch_set_stream", "acs_batch_set_field", "acs_batch_get_field",
+    "acs_batch_set_fields", "acs_batch_get_fields",
     "acs_batch_run", "acs_batch_launch_count", "acs_launch_count", "acs_batch_time_kernel",
     "acs_batch_set_option", "acs_set_option", "acs_solve_u_static",
     "acs_batch_ws_enable", "acs_batch_ws_features", "acs_batch_ws_target", "acs_batch_set_start",
@@ -126,6 +127,8 @@ def _declare(L):
     L.acs_batch_set_stream.argtypes = [V, V]
     L.acs_batch_set_field.argtypes = [V, C.c_int, C.c_int, _D]
     L.acs_batch_get_field.argtypes = [V, C.c_int, C.c_int, _D]
+    L.acs_batch_set_fields.argtypes = [V, C.c_int, C.c_int, _I, C.POINTER(_D)]
+    L.acs_batch_get_fields.argtypes = [V, C.c_int, C.c_int, _I, C.POINTER(_D)]
     L.acs_batch_run.argtypes = [V, C.c_int, _I, _I, _D, _I]
     L.acs_batch_launch_count.argtypes = [V, C.POINTER(C.c_longlong)]
     L.acs_launch_count.argtypes = [V, C.POINTER(C.c_longlong)]
@@ -397,17 +400,20 @@ class Batch:
         return np.zeros(field_shape(name, p.imax, p.jmax), order="F")
 
     def set_state(self, c: int, state: dict):
-        for n, a in state.items():
-            _check(lib().acs_batch_set_field(self.h, c, FIELD_ID[n], _dp(np.asfortranarray(a))),
-                   "acs_batch_set_field")
+        if not state:
+            return
+        arrs = [np.asfortranarray(a) for a in state.values()]
+        ids = (C.c_int * len(arrs))(*[FIELD_ID[n] for n in state])
+        _check(lib().acs_batch_set_fields(self.h, c, len(arrs), ids, (_D * len(arrs))(*[_dp(a) for a in arrs])),
+               "acs_batch_set_fields")
 
     def get_state(self, c: int, names=FIELDS, out=None) -> dict:
         """Download fields of case c (into the arrays of `out` when given)."""
-        res = {}
-        for n in names:
-            a = out[n] if out is not None else self.zeros(c, n)
-            _check(lib().acs_batch_get_field(self.h, c, FIELD_ID[n], _dp(a)), "acs_batch_get_field")
-            res[n] = a
+        res = {n: out[n] if out is not None else self.zeros(c, n) for n in names}
+        if res:
+            ids = (C.c_int * len(res))(*[FIELD_ID[n] for n in res])
+            _check(lib().acs_batch_get_fields(self.h, c, len(res), ids, (_D * len(res))(*[_dp(a) for a in res.values()])),
+                   "acs_batch_get_fields")
         return res
 
     def run(self, n_steps: int, itc):

@@ -25,6 +25,7 @@
 #include "engine_api.h"
 #include "kernels.h"
 #include "tile_engine.h"
+#include "transfer.h"
 #include "warmstart.h"
 
 namespace acs {
@@ -90,6 +91,10 @@ struct Batch {
   int* d_iters = nullptr;
   double* d_err = nullptr;
   long long stats_cap = 0;
+  bool ctl_stale = false;     // hk holds changes that the device's control words do not have yet
+  double* d_stage = nullptr;  // staging of field transfers: device, and pinned host for per-routine calls
+  double* h_stage = nullptr;
+  size_t d_stage_cap = 0, h_stage_cap = 0;  // doubles
   int* h_flag = nullptr;  // mapped host word for the host-polled loop
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -148,6 +153,8 @@ struct Batch {
     if (pool) cudaFree(pool);
     if (d_iters) cudaFree(d_iters);
     if (d_err) cudaFree(d_err);
+    if (d_stage) cudaFree(d_stage);
+    if (h_stage) cudaFreeHost(h_stage);
     if (h_flag) cudaFreeHost(h_flag);
     if (d_cases) cudaFree(d_cases);
     if (d_tetiles) cudaFree(d_tetiles);
@@ -245,22 +252,35 @@ int field_dims(const CaseDev& d, int family, int* w, int* h) {
   return 0;
 }
 
-int put(Batch& b, int c, int family, int idx, const double* host) {
-  const CaseDev& d = b.hc[c];
-  int w, h;
-  field_dims(d, family, &w, &h);
-  CU(cudaMemcpy2DAsync(b.buf(c, family, idx), (size_t)d.pitch * 8, host, (size_t)w * 8, (size_t)w * 8, h,
-                       cudaMemcpyHostToDevice, b.stream));
+// Staging buffers of at least n doubles, kept with the batch.
+int stage_dev(Batch& b, size_t n) {
+  if (n <= b.d_stage_cap) return ACS_OK;
+  CU(cudaStreamSynchronize(b.stream));
+  if (b.d_stage) cudaFree(b.d_stage);
+  b.d_stage = nullptr;
+  b.d_stage_cap = 0;
+  CU(cudaMalloc(&b.d_stage, n * sizeof(double)));
+  b.d_stage_cap = n;
+  return ACS_OK;
+}
+int stage_host(Batch& b, size_t n) {
+  if (n <= b.h_stage_cap) return ACS_OK;
+  if (b.h_stage) cudaFreeHost(b.h_stage);
+  b.h_stage = nullptr;
+  b.h_stage_cap = 0;
+  CU(cudaMallocHost(&b.h_stage, n * sizeof(double)));
+  b.h_stage_cap = n;
   return ACS_OK;
 }
 
-int get(Batch& b, int c, int family, int idx, double* host) {
+// Adds a field of case c to a list of transfers.
+void add_move(const Batch& b, MoveList& m, int c, int family, int idx) {
   const CaseDev& d = b.hc[c];
   int w, h;
   field_dims(d, family, &w, &h);
-  CU(cudaMemcpy2DAsync(host, (size_t)w * 8, b.buf(c, family, idx), (size_t)d.pitch * 8, (size_t)w * 8, h,
-                       cudaMemcpyDeviceToHost, b.stream));
-  return ACS_OK;
+  m.f[m.n++] = FieldMove{b.buf(c, family, idx), m.total, w, h};
+  m.pitch = d.pitch;
+  m.total += (long long)w * h;
 }
 
 bool all_ones(const double* a, size_t n) {
@@ -269,13 +289,14 @@ bool all_ones(const double* a, size_t n) {
   return true;
 }
 
-int upload_field(Batch& b, int c, int field, const double* host) {
+// Before field `field` of case c is overwritten: control changes and copies that its role needs.
+// Returns the field's place in *L.
+int prepare_upload(Batch& b, int c, int field, const double* host, FieldLoc* out) {
   FieldLoc L = field_loc(field);
   if (L.family < 0) return fail(ACS_E_ARG, "unknown field id");
   if (field == ACS_UM_TAU || field == ACS_VM_TAU) {
     b.hk[c].tau_dirty = 1;
-    int r = push_ctl(b);
-    if (r) return r;
+    b.ctl_stale = true;
   }
   if (L.role == R_NTAU && L.family != 2 && b.hk[c].ntau_alias) {
     // give every n_tau array its own values again before one of them is overwritten
@@ -291,8 +312,7 @@ int upload_field(Batch& b, int c, int field, const double* host) {
                          cudaMemcpyDeviceToDevice, b.stream));
     }
     k.ntau_alias = 0;
-    int r = push_ctl(b);
-    if (r) return r;
+    b.ctl_stale = true;
   }
   if (L.family == 2) {
     // p and pn share one buffer after a non-exit iteration; give pn its own buffer first
@@ -301,19 +321,51 @@ int upload_field(Batch& b, int c, int field, const double* host) {
       const CaseDev& d = b.hc[c];
       CU(cudaMemcpyAsync(d.P[k.rp[1]], d.P[k.rp[0]], sizeof(double) * d.n_elems, cudaMemcpyDeviceToDevice, b.stream));
       k.rp_read = k.rp[1];
-      int r = push_ctl(b);
-      if (r) return r;
+      b.ctl_stale = true;
     }
   }
   if (field == ACS_T) b.t_unity[c] = all_ones(host, (size_t)b.hc[c].nx * b.hc[c].ny);
-  return put(b, c, L.family, b.role_index(c, L), host);
+  *out = L;
+  return ACS_OK;
 }
 
-int download_field(Batch& b, int c, int field, double* host) {
-  FieldLoc L = field_loc(field);
-  if (L.family < 0) return fail(ACS_E_ARG, "unknown field id");
-  int r = get(b, c, L.family, b.role_index(c, L), host);
+// n distinct fields of case c from contiguous host arrays, each applied in the order given.
+int upload_fields(Batch& b, int c, int n, const int* fields, const double* const* host) {
+  MoveList m{};
+  for (int q = 0; q < n; ++q) {
+    const FieldLoc l = field_loc(fields[q]);
+    if (q && l.role == R_NTAU && l.family >= 0 && l.family != 2 && b.hk[c].ntau_alias) {
+      // n_tau arrays get their own copies now, of what the fields before this one have become
+      int r = upload_fields(b, c, q, fields, host);
+      return r ? r : upload_fields(b, c, n - q, fields + q, host + q);
+    }
+    FieldLoc L;
+    int r = prepare_upload(b, c, fields[q], host[q], &L);
+    if (r) return r;
+    add_move(b, m, c, L.family, b.role_index(c, L));
+  }
+  int r = stage_dev(b, (size_t)m.total);
   if (r) return r;
+  for (int q = 0; q < n; ++q)
+    CU(cudaMemcpyAsync(b.d_stage + m.f[q].off, host[q], sizeof(double) * m.f[q].w * m.f[q].h, cudaMemcpyHostToDevice, b.stream));
+  move_to_case(m, b.d_stage, nullptr, CaseCtl{}, b.stream);
+  CU(cudaGetLastError());
+  return ACS_OK;
+}
+
+int download_fields(Batch& b, int c, int n, const int* fields, double* const* host) {
+  MoveList m{};
+  for (int q = 0; q < n; ++q) {
+    FieldLoc L = field_loc(fields[q]);
+    if (L.family < 0) return fail(ACS_E_ARG, "unknown field id");
+    add_move(b, m, c, L.family, b.role_index(c, L));
+  }
+  int r = stage_dev(b, (size_t)m.total);
+  if (r) return r;
+  move_from_case(m, b.d_stage, nullptr, b.stream);
+  CU(cudaGetLastError());
+  for (int q = 0; q < n; ++q)
+    CU(cudaMemcpyAsync(host[q], b.d_stage + m.f[q].off, sizeof(double) * m.f[q].w * m.f[q].h, cudaMemcpyDeviceToHost, b.stream));
   CU(cudaStreamSynchronize(b.stream));
   return ACS_OK;
 }
@@ -333,9 +385,12 @@ int refresh_flags(Batch& b) {
 }
 
 int push_ctl(Batch& b) {
+  b.ctl_stale = false;
   CU(cudaMemcpyAsync(b.dk, b.hk.data(), sizeof(CaseCtl) * b.n, cudaMemcpyHostToDevice, b.stream));
   return ACS_OK;
 }
+// before kernels that read the control words outside a run
+int flush_ctl(Batch& b) { return b.ctl_stale ? push_ctl(b) : ACS_OK; }
 int pull_ctl(Batch& b) {
   CU(cudaMemcpyAsync(b.hk.data(), b.dk, sizeof(CaseCtl) * b.n, cudaMemcpyDeviceToHost, b.stream));
   CU(cudaStreamSynchronize(b.stream));
@@ -963,24 +1018,47 @@ int run_engine(Batch& b) {
   return ACS_OK;
 }
 
-// Per-routine calls run one routine's launches on case 0 with identity roles.
-int begin_routine(Batch& b) {
+// Per-routine calls run one routine's launches on case 0 with identity roles.  The driver's arrays
+// cross PCIe in one copy each way through pinned staging, the control word travels with them, and the host
+// waits once.
+struct RoutineIO { int family, role; const double* in; double* out; };
+
+int begin_routine(Batch& b, const RoutineIO* io, int n) {
   CaseCtl& k = b.hk[0];
   reset_roles(k);
   k.active = 1;
   k.scalars = 1;
   k.res_u = k.res_v = k.res_p = 0;
-  return push_ctl(b);
+  MoveList m{};
+  for (int q = 0; q < n; ++q) add_move(b, m, 0, io[q].family, io[q].role);
+  int r = stage_dev(b, (size_t)m.total + 4);
+  if (!r) r = stage_host(b, (size_t)m.total + 4);
+  if (r) return r;
+  for (int q = 0; q < n; ++q) std::memcpy(b.h_stage + m.f[q].off, io[q].in, sizeof(double) * m.f[q].w * m.f[q].h);
+  CU(cudaMemcpyAsync(b.d_stage, b.h_stage, sizeof(double) * m.total, cudaMemcpyHostToDevice, b.stream));
+  move_to_case(m, b.d_stage, b.dk, k, b.stream);
+  CU(cudaGetLastError());
+  b.ctl_stale = false;
+  return ACS_OK;
 }
 
-int end_routine(Batch& b) {
-  CU(cudaStreamSynchronize(b.stream));
+int end_routine(Batch& b, const RoutineIO* io, int n) {
+  MoveList m{};
+  for (int q = 0; q < n; ++q) add_move(b, m, 0, io[q].family, io[q].role);
+  int r = stage_dev(b, (size_t)m.total + 4);
+  if (!r) r = stage_host(b, (size_t)m.total + 4);
+  if (r) return r;
+  move_from_case(m, b.d_stage, b.dk, b.stream);
   CU(cudaGetLastError());
-  int r = pull_ctl(b);
-  b.hk[0].active = 0;
-  if (!r) r = push_ctl(b);
-  if (!r) CU(cudaStreamSynchronize(b.stream));
-  return r;
+  CU(cudaMemcpyAsync(b.h_stage, b.d_stage, sizeof(double) * (m.total + 3), cudaMemcpyDeviceToHost, b.stream));
+  CU(cudaStreamSynchronize(b.stream));
+  for (int q = 0; q < n; ++q) std::memcpy(io[q].out, b.h_stage + m.f[q].off, sizeof(double) * m.f[q].w * m.f[q].h);
+  CaseCtl& k = b.hk[0];
+  std::memcpy(&k.res_u, b.h_stage + m.total, 8);
+  std::memcpy(&k.res_v, b.h_stage + m.total + 1, 8);
+  std::memcpy(&k.res_p, b.h_stage + m.total + 2, 8);
+  k.active = 0;
+  return ACS_OK;
 }
 
 double bits_to_double(unsigned long long v) {
@@ -1044,13 +1122,29 @@ int acs_batch_set_stream(acs_batch* h, void* s) {
 int acs_batch_set_field(acs_batch* h, int c, int field, const double* host) {
   if (!h || !host) return acs::fail(ACS_E_ARG, "null argument");
   if (c < 0 || c >= h->b->n) return acs::fail(ACS_E_ARG, "case id out of range");
-  return acs::upload_field(*h->b, c, field, host);
+  return acs::upload_fields(*h->b, c, 1, &field, &host);
+}
+
+int acs_batch_set_fields(acs_batch* h, int c, int n, const int* fields, const double* const* host) {
+  if (!h || !fields || !host || n < 1 || n > acs::MOVE_MAX) return acs::fail(ACS_E_ARG, "bad argument");
+  if (c < 0 || c >= h->b->n) return acs::fail(ACS_E_ARG, "case id out of range");
+  for (int q = 0; q < n; ++q)
+    if (!host[q]) return acs::fail(ACS_E_ARG, "null argument");
+  return acs::upload_fields(*h->b, c, n, fields, host);
 }
 
 int acs_batch_get_field(acs_batch* h, int c, int field, double* host) {
   if (!h || !host) return acs::fail(ACS_E_ARG, "null argument");
   if (c < 0 || c >= h->b->n) return acs::fail(ACS_E_ARG, "case id out of range");
-  return acs::download_field(*h->b, c, field, host);
+  return acs::download_fields(*h->b, c, 1, &field, &host);
+}
+
+int acs_batch_get_fields(acs_batch* h, int c, int n, const int* fields, double* const* host) {
+  if (!h || !fields || !host || n < 1 || n > acs::MOVE_MAX) return acs::fail(ACS_E_ARG, "bad argument");
+  if (c < 0 || c >= h->b->n) return acs::fail(ACS_E_ARG, "case id out of range");
+  for (int q = 0; q < n; ++q)
+    if (!host[q]) return acs::fail(ACS_E_ARG, "null argument");
+  return acs::download_fields(*h->b, c, n, fields, host);
 }
 
 int acs_batch_cell_fields(acs_batch* h, int c, double* u, double* v, double* vel_mag) {
@@ -1115,6 +1209,7 @@ int acs_batch_ws_features(acs_batch* h, float* X, float* inc_scale) {
   if (!h || !X) return acs::fail(ACS_E_ARG, "null argument");
   Batch& b = *h->b;
   if (!b.ws_pool) return acs::fail(ACS_E_STATE, "warm start not enabled");
+  if (int r = acs::flush_ctl(b)) return r;
   acs::launch_ws_features(b.dc, b.dk, b.d_ws, b.n, b.ws_H, b.ws_W, b.ws_has_prev, b.d_ws_ss, b.d_ws_sc, X, inc_scale,
                           b.stream);
   CU(cudaGetLastError());
@@ -1127,6 +1222,7 @@ int acs_batch_ws_target(acs_batch* h, float* T, float* Wt) {
   if (!h || !T || !Wt) return acs::fail(ACS_E_ARG, "null argument");
   Batch& b = *h->b;
   if (!b.ws_pool) return acs::fail(ACS_E_STATE, "warm start not enabled");
+  if (int r = acs::flush_ctl(b)) return r;
   acs::launch_ws_target(b.dc, b.dk, b.d_ws, b.n, b.ws_H, b.ws_W, b.d_ws_sc, T, Wt, b.stream);
   CU(cudaGetLastError());
   return ACS_OK;
@@ -1140,6 +1236,7 @@ int acs_batch_set_start(acs_batch* h, const float* Y, int ldy, const float* scal
   if (policy < 0 || policy > 2) return acs::fail(ACS_E_ARG, "policy must be 0, 1 or 2");
   if (Y && (!scale || ldy < acs::WS_FIELDS)) return acs::fail(ACS_E_ARG, "Y needs scale and ldy >= 5");
   // the quadratic candidate needs two increments, i.e. three feature calls; before that, linear
+  if (int r = acs::flush_ctl(b)) return r;
   const int order = (b.ws_order == 2 && b.ws_calls >= 3) ? 2 : 1;
   acs::launch_ws_start(b.dc, b.dk, b.d_ws, b.n, b.ws_H, b.ws_W, b.d_ws_sc, Y, ldy, scale, policy, order,
                        b.d_ws_res, b.d_ws_choice, b.stream);
@@ -1330,12 +1427,12 @@ int acs_set_stream(acs_handle* h, void* s) {
 
 int acs_set_field(acs_handle* h, int field, const double* host) {
   if (!h || !host) return acs::fail(ACS_E_ARG, "null argument");
-  return acs::upload_field(*h->b, 0, field, host);
+  return acs::upload_fields(*h->b, 0, 1, &field, &host);
 }
 
 int acs_get_field(acs_handle* h, int field, double* host) {
   if (!h || !host) return acs::fail(ACS_E_ARG, "null argument");
-  return acs::download_field(*h->b, 0, field, host);
+  return acs::download_fields(*h->b, 0, 1, &field, &host);
 }
 
 int acs_cell_fields(acs_handle* h, double* u, double* v, double* vel_mag) {
@@ -1364,18 +1461,15 @@ int acs_solve_u(acs_handle* h, const double* um, const double* um_tau, double* v
                 double* um_n_tau, double* residual_u) {
   NEED(h); NEED(um); NEED(um_tau); NEED(vm_tau); NEED(p); NEED(um_n_tau); NEED(residual_u);
   Batch& b = *h->b;
+  const acs::RoutineIO in[4] = {{0, acs::R_PHYS, um, nullptr}, {0, acs::R_TAU, um_tau, nullptr},
+                                {1, acs::R_TAU, vm_tau, nullptr}, {2, 1, p, nullptr}};
+  const acs::RoutineIO out[2] = {{0, acs::R_NTAU, nullptr, um_n_tau}, {1, acs::R_TAU, nullptr, vm_tau}};
   int r = acs::refresh_flags(b);
-  if (!r) r = acs::begin_routine(b);
-  if (!r) r = acs::put(b, 0, 0, acs::R_PHYS, um);
-  if (!r) r = acs::put(b, 0, 0, acs::R_TAU, um_tau);
-  if (!r) r = acs::put(b, 0, 1, acs::R_TAU, vm_tau);
-  if (!r) r = acs::put(b, 0, 2, 1, p);
+  if (!r) r = acs::begin_routine(b, in, 4);
   if (r) return r;
   acs::seq_u(b);
-  r = acs::end_routine(b);
-  if (!r) r = acs::get(b, 0, 0, acs::R_NTAU, um_n_tau);
-  if (!r) r = acs::get(b, 0, 1, acs::R_TAU, vm_tau);
-  if (!r) { cudaStreamSynchronize(b.stream); *residual_u = acs::bits_to_double(b.hk[0].res_u); }
+  r = acs::end_routine(b, out, 2);
+  if (!r) *residual_u = acs::bits_to_double(b.hk[0].res_u);
   return r;
 }
 
@@ -1383,20 +1477,16 @@ int acs_solve_v(acs_handle* h, const double* vm, double* um_tau, const double* v
                 const double* T, double* vm_n_tau, double* residual_v) {
   NEED(h); NEED(vm); NEED(um_tau); NEED(vm_tau); NEED(p); NEED(T); NEED(vm_n_tau); NEED(residual_v);
   Batch& b = *h->b;
+  const acs::RoutineIO in[5] = {{1, acs::R_PHYS, vm, nullptr}, {0, acs::R_TAU, um_tau, nullptr},
+                                {1, acs::R_TAU, vm_tau, nullptr}, {2, 1, p, nullptr}, {3, acs::R_PHYS, T, nullptr}};
+  const acs::RoutineIO out[2] = {{1, acs::R_NTAU, nullptr, vm_n_tau}, {0, acs::R_TAU, nullptr, um_tau}};
   b.t_unity[0] = acs::all_ones(T, (size_t)b.hc[0].nx * b.hc[0].ny);
   int r = acs::refresh_flags(b);
-  if (!r) r = acs::begin_routine(b);
-  if (!r) r = acs::put(b, 0, 1, acs::R_PHYS, vm);
-  if (!r) r = acs::put(b, 0, 0, acs::R_TAU, um_tau);
-  if (!r) r = acs::put(b, 0, 1, acs::R_TAU, vm_tau);
-  if (!r) r = acs::put(b, 0, 2, 1, p);
-  if (!r) r = acs::put(b, 0, 3, acs::R_PHYS, T);
+  if (!r) r = acs::begin_routine(b, in, 5);
   if (r) return r;
   acs::seq_v(b);
-  r = acs::end_routine(b);
-  if (!r) r = acs::get(b, 0, 1, acs::R_NTAU, vm_n_tau);
-  if (!r) r = acs::get(b, 0, 0, acs::R_TAU, um_tau);
-  if (!r) { cudaStreamSynchronize(b.stream); *residual_v = acs::bits_to_double(b.hk[0].res_v); }
+  r = acs::end_routine(b, out, 2);
+  if (!r) *residual_v = acs::bits_to_double(b.hk[0].res_v);
   return r;
 }
 
@@ -1404,15 +1494,13 @@ int acs_solve_p(acs_handle* h, const double* p, const double* um_n_tau, const do
                 double* residual_p) {
   NEED(h); NEED(p); NEED(um_n_tau); NEED(vm_n_tau); NEED(pn); NEED(residual_p);
   Batch& b = *h->b;
-  int r = acs::begin_routine(b);
-  if (!r) r = acs::put(b, 0, 2, 0, p);
-  if (!r) r = acs::put(b, 0, 0, acs::R_NTAU, um_n_tau);
-  if (!r) r = acs::put(b, 0, 1, acs::R_NTAU, vm_n_tau);
+  const acs::RoutineIO in[3] = {{2, 0, p, nullptr}, {0, acs::R_NTAU, um_n_tau, nullptr}, {1, acs::R_NTAU, vm_n_tau, nullptr}};
+  const acs::RoutineIO out[1] = {{2, 1, nullptr, pn}};
+  int r = acs::begin_routine(b, in, 3);
   if (r) return r;
   acs::seq_p(b);
-  r = acs::end_routine(b);
-  if (!r) r = acs::get(b, 0, 2, 1, pn);
-  if (!r) { cudaStreamSynchronize(b.stream); *residual_p = acs::bits_to_double(b.hk[0].res_p); }
+  r = acs::end_routine(b, out, 1);
+  if (!r) *residual_p = acs::bits_to_double(b.hk[0].res_p);
   return r;
 }
 
@@ -1421,17 +1509,13 @@ static int solve_scalar(acs_handle* h, bool is_c, const double* um_n_tau, const 
   NEED(h); NEED(um_n_tau); NEED(vm_n_tau); NEED(Z); NEED(Z_n_tau); NEED(Z_tau);
   Batch& b = *h->b;
   const int fam = is_c ? 4 : 3;
-  int r = acs::begin_routine(b);
-  if (!r) r = acs::put(b, 0, 0, acs::R_NTAU, um_n_tau);
-  if (!r) r = acs::put(b, 0, 1, acs::R_NTAU, vm_n_tau);
-  if (!r) r = acs::put(b, 0, fam, acs::R_PHYS, Z);
-  if (!r) r = acs::put(b, 0, fam, acs::R_TAU, Z_tau);
+  const acs::RoutineIO in[4] = {{0, acs::R_NTAU, um_n_tau, nullptr}, {1, acs::R_NTAU, vm_n_tau, nullptr},
+                                {fam, acs::R_PHYS, Z, nullptr}, {fam, acs::R_TAU, Z_tau, nullptr}};
+  const acs::RoutineIO out[1] = {{fam, acs::R_NTAU, nullptr, Z_n_tau}};
+  int r = acs::begin_routine(b, in, 4);
   if (r) return r;
   acs::seq_s(b, is_c);
-  r = acs::end_routine(b);
-  if (!r) r = acs::get(b, 0, fam, acs::R_NTAU, Z_n_tau);
-  if (!r) { cudaError_t e = cudaStreamSynchronize(b.stream); if (e != cudaSuccess) return acs::fail(ACS_E_CUDA, cudaGetErrorString(e)); }
-  return r;
+  return acs::end_routine(b, out, 1);
 }
 
 int acs_solve_z(acs_handle* h, const double* um_n_tau, const double* vm_n_tau, const double* T, double* T_n_tau,
