@@ -13,10 +13,14 @@
 //     and itc=0 (main.f90:154-157,182) -> swap the phys and n_tau roles;
 //   * the loop condition itc < itc_max fails after the copies (main.f90:120): the latest iterate
 //     is then in the tau buffers and is copied into phys.
+// The last block to finish also ends the loop body: it sets the WHILE condition of the graph (continue
+// while any case is active, bounded by max_iters pseudo-iterations so the loop always ends), or publishes the
+// number of active cases to a mapped host word for the host-polled loop.
 // A NaN or infinite residual marks the case FAILED and removes it from the launch (the reference
 // would run on to itc_max).
 #include <cuda_runtime.h>
 #include "acs_dev.cuh"
+#include "bc_exact.cuh"
 #include "kernels.h"
 
 namespace acs {
@@ -24,11 +28,18 @@ namespace acs {
 __device__ inline void swap_i(int& a, int& b) { int t = a; a = b; b = t; }
 
 __global__ void k_control(const CaseDev* __restrict__ cs, CaseCtl* __restrict__ ctl, int* iters,
-                          double* err, int* n_active) {
+                          double* err, int* n_active, LoopEnd end) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched while the iteration's last kernel drains
   const int c = blockIdx.x;
   CaseCtl& k = ctl[c];
   const CaseDev& d = cs[c];
   __shared__ int s_copy;
+  if (end.tau_bc && k.active && k.tau_dirty) {
+    // the first iteration after an upload: the boundary passes' side effect on um_tau and vm_tau, which
+    // the tile kernels of the iteration applied to their own copies
+    bc_uv_block(d, d.U[k.ru[R_TAU]], d.V[k.rv[R_TAU]]);
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
     s_copy = 0;
     if (k.active) {
@@ -91,6 +102,18 @@ __global__ void k_control(const CaseDev* __restrict__ cs, CaseCtl* __restrict__ 
       }
       if (k.active) atomicAdd(n_active, 1);
     }
+    if (end.mode != LOOP_NONE) {
+      // the block that finishes last counts the iteration and decides whether another follows
+      __threadfence();
+      if (atomicAdd(end.ticket, 1) == (int)gridDim.x - 1) {
+        __threadfence();
+        *end.ticket = 0;
+        const int a = atomicExch(n_active, 0);
+        const long long it = ++*end.iter_count;
+        if (end.mode == LOOP_COND) cudaGraphSetConditional(end.handle, (a > 0 && it < end.max_iters) ? 1u : 0u);
+        else *(volatile int*)end.host_flag = a;
+      }
+    }
   }
   __syncthreads();
   if (s_copy) {
@@ -101,24 +124,6 @@ __global__ void k_control(const CaseDev* __restrict__ cs, CaseCtl* __restrict__ 
     for (int f = 0; f < nf; ++f)
       for (long long q = threadIdx.x; q < n; q += blockDim.x) dst[f][q] = src[f][q];
   }
-}
-
-// Sets the WHILE condition of the graph: continue while any case is active, bounded by
-// max_iters pseudo-iterations so the loop always ends.
-__global__ void k_loop_cond(int* n_active, long long* iter_count, long long max_iters,
-                            cudaGraphConditionalHandle handle) {
-  const int a = *n_active;
-  *n_active = 0;
-  const long long it = ++(*iter_count);
-  cudaGraphSetConditional(handle, (a > 0 && it < max_iters) ? 1u : 0u);
-}
-
-// Host-polled variant: publishes the number of active cases to a mapped host word.
-__global__ void k_loop_flag(int* n_active, long long* iter_count, int* host_flag) {
-  const int a = *n_active;
-  *n_active = 0;
-  ++(*iter_count);
-  *(volatile int*)host_flag = a;
 }
 
 }  // namespace acs

@@ -25,9 +25,16 @@ cudaError_t launch_cell_fields(const double* um, const double* vm, int nx, int n
                                double* mag, cudaStream_t s);
 
 // loop control (control.cu)
-__global__ void k_control(const CaseDev*, CaseCtl*, int* iters, double* err, int* n_active);
-__global__ void k_loop_cond(int* n_active, long long* iter_count, long long max_iters,
-                            cudaGraphConditionalHandle handle);
-__global__ void k_loop_flag(int* n_active, long long* iter_count, int* host_flag);
+enum LoopMode { LOOP_NONE = 0, LOOP_COND = 1, LOOP_FLAG = 2 };
+struct LoopEnd {
+  int mode;                           // what the last block does with the number of active cases
+  int tau_bc;                         // 1: apply the first iteration's side effects on um_tau, vm_tau
+  cudaGraphConditionalHandle handle;  // LOOP_COND
+  long long max_iters;
+  long long* iter_count;
+  int* ticket;                        // blocks done (0 between launches)
+  int* host_flag;                     // LOOP_FLAG
+};
+__global__ void k_control(const CaseDev*, CaseCtl*, int* iters, double* err, int* n_active, LoopEnd end);
 
 }  // namespace acs

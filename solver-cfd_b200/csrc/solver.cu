@@ -101,6 +101,7 @@ struct Batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   bool graph_conditional = true;
+  bool overlap = true;  // tile engine: programmatic dependent launches inside the loop body
   bool use_fast = false;
   FastPlan* fast = nullptr;
   long long launches = 0;
@@ -628,8 +629,8 @@ void launch_timed_kernel(Batch& b, int kernel) {
     case 2: (b.use_fast ? launch_p_fast : launch_p_exact)(b.dc, b.dk, b.dtiles, b.ntiles, b.stream); break;
     case 3: (b.use_fast ? launch_s_stage_fast : launch_s_stage_exact)(false, 1, b.dc, b.dk, b.dtiles, b.ntiles, b.stream); break;
     case 4: (b.use_fast ? launch_s_stage_fast : launch_s_stage_exact)(true, 1, b.dc, b.dk, b.dtiles, b.ntiles, b.stream); break;
-    case 5: te_launch_uv(2, b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.stream); break;
-    case 6: te_launch_ptc(b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.stream); break;
+    case 5: te_launch_uv(2, b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, false, b.stream); break;
+    case 6: te_launch_ptc(b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, false, b.stream); break;
   }
 }
 
@@ -660,19 +661,42 @@ int te_setup(Batch& b) {
   return ACS_OK;
 }
 
+// What k_control's last block does at the end of an iteration (mode, handle, max_iters, host flag set by
+// build_graph).
+LoopEnd loop_end(Batch& b, int mode) {
+  LoopEnd e{};
+  e.mode = mode;
+  e.tau_bc = b.engine == 2;
+  e.iter_count = b.d_iter;
+  e.ticket = b.d_nactive + 32;
+  return e;
+}
+
+void launch_control(Batch& b, const LoopEnd& end) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(b.n);
+  cfg.blockDim = dim3(256);
+  cfg.stream = b.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = b.engine == 2 && b.overlap ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_control, (const CaseDev*)b.dc, b.dk, b.d_iters, b.d_err, b.d_nactive, end);
+  b.launches += 1;
+}
+
 // one pseudo-iteration of the tile engine: U/V stages 1-3, P + T/C, control
-void te_iteration(Batch& b) {
-  for (int s = 1; s <= 3; ++s) {
-    te_launch_uv(s, b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.stream);
-    if (s == 1) te_launch_tau_bc(b.dc, b.dk, b.n, b.stream);
-  }
-  te_launch_ptc(b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.stream);
-  k_control<<<b.n, 256, 0, b.stream>>>(b.dc, b.dk, b.d_iters, b.d_err, b.d_nactive);
-  b.launches += 6;
+void te_iteration(Batch& b, const LoopEnd& end) {
+  for (int s = 1; s <= 3; ++s)
+    te_launch_uv(s, b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.overlap && s > 1, b.stream);
+  te_launch_ptc(b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.overlap, b.stream);
+  b.launches += 4;
+  launch_control(b, end);
 }
 
 // one pseudo-iteration (main.f90:122-150) for every active case
-void seq_iteration(Batch& b) {
+void seq_iteration(Batch& b, const LoopEnd& end) {
   seq_u(b);
   seq_v(b);
   seq_p(b);
@@ -680,8 +704,7 @@ void seq_iteration(Batch& b) {
     seq_s(b, false);
     seq_s(b, true);
   }
-  k_control<<<b.n, 256, 0, b.stream>>>(b.dc, b.dk, b.d_iters, b.d_err, b.d_nactive);
-  b.launches += 1;
+  launch_control(b, end);
 }
 
 long long max_total_iterations(const Batch& b, int n_steps) {
@@ -714,10 +737,12 @@ int build_graph(Batch& b, int n_steps) {
       e = cudaStreamBeginCaptureToGraph(b.stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
         const long long l0 = b.launches;
-        if (b.engine == 2) te_iteration(b);
-        else seq_iteration(b);
-        k_loop_cond<<<1, 1, 0, b.stream>>>(b.d_nactive, b.d_iter, max_total_iterations(b, n_steps), h);
-        b.body_kernels = b.launches - l0 + 1;
+        LoopEnd end = loop_end(b, LOOP_COND);
+        end.handle = h;
+        end.max_iters = max_total_iterations(b, n_steps);
+        if (b.engine == 2) te_iteration(b, end);
+        else seq_iteration(b, end);
+        b.body_kernels = b.launches - l0;
         e = cudaStreamEndCapture(b.stream, &body);
       }
     }
@@ -729,6 +754,11 @@ int build_graph(Batch& b, int n_steps) {
     }
     cudaGetLastError();
     cudaGraphDestroy(g);
+    b.launches = saved;
+    if (b.engine == 2 && b.overlap) {  // once more without overlapped launches
+      b.overlap = false;
+      return build_graph(b, n_steps);
+    }
     b.graph_conditional = false;  // fall back to the host-polled loop below
   }
   // host-polled: the graph holds one iteration plus a flag publish
@@ -738,10 +768,11 @@ int build_graph(Batch& b, int n_steps) {
   cudaGraph_t g;
   CU(cudaStreamBeginCapture(b.stream, cudaStreamCaptureModeThreadLocal));
   const long long l0 = b.launches;
-  if (b.engine == 2) te_iteration(b);
-  else seq_iteration(b);
-  k_loop_flag<<<1, 1, 0, b.stream>>>(b.d_nactive, b.d_iter, d_flag);
-  b.body_kernels = b.launches - l0 + 1;
+  LoopEnd end = loop_end(b, LOOP_FLAG);
+  end.host_flag = d_flag;
+  if (b.engine == 2) te_iteration(b, end);
+  else seq_iteration(b, end);
+  b.body_kernels = b.launches - l0;
   CU(cudaStreamEndCapture(b.stream, &g));
   CU(cudaGraphInstantiate(&b.gexec, g, 0));
   b.graph = g;
