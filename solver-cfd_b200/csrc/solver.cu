@@ -1142,6 +1142,11 @@ int acs_batch_set_stream(acs_batch* h, void* s) {
   Batch& b = *h->b;
   if (b.gexec) { cudaGraphExecDestroy(b.gexec); b.gexec = nullptr; }
   if (b.graph) { cudaGraphDestroy(b.graph); b.graph = nullptr; }
+  // transfers on the stream so far may still use the staging buffer: it is freed (which waits for them),
+  // and the new stream's first transfer makes its own
+  if (b.d_stage) cudaFree(b.d_stage);
+  b.d_stage = nullptr;
+  b.d_stage_cap = 0;
   if (s) {
     if (b.own_stream) cudaStreamDestroy(b.stream);
     b.stream = (cudaStream_t)s;
