@@ -536,7 +536,9 @@ __global__ void __launch_bounds__(CHIP_THREADS, 1) k_chip(ChipArgs a) {
   // vm(imax, jmax+1) of the reference variant: bcUV's row pass computes it from what the n_tau
   // array holds in column imax before its column pass, i.e. from that array's previous contents
   // (the loop never reads it).  The stage windows rotate differently from the case's buffers, so
-  // that history is kept here: nodes (imax, jmax-1) and (imax, jmax-2) of the buffer in each role.
+  // that history is kept here: nodes (imax, jmax-1) and (imax, jmax-2) of the buffer in each role.  (The tile
+  // engine's n_tau tile holds the physical-step array before its passes; a batch that runs here in its
+  // place gets the value from that one.)
   const bool corner = d.bc == 0 && r1 == R + 1 && tid == 0;
   double h1[3] = {0, 0, 0}, h2[3] = {0, 0, 0};
   if (corner)
@@ -621,14 +623,14 @@ __global__ void __launch_bounds__(CHIP_THREADS, 1) k_chip(ChipArgs a) {
         ph = 1;
       } else {
         if (corner) {
-          // (imax, jmax+1) of vm_n_tau from the n_tau buffer's history, then that history's update
+          // (imax, jmax+1) of vm_n_tau from the buffers' history, then the n_tau buffer's update
           if (dirty) {
             h1[R_TAU] = V(ut)[at(nx, ny - 1)];
             h2[R_TAU] = V(ut)[at(nx, ny - 2)];
           }
           double* vn = V(ua);
-          const double n = 2.0 * h2[R_NTAU] - h1[R_NTAU];
-          vn[at(nx, ny + 1)] = 2.0 * h1[R_NTAU] - n;
+          const double c1 = h1[a.corner_role], c2 = h2[a.corner_role], n = 2.0 * c2 - c1;
+          vn[at(nx, ny + 1)] = 2.0 * c1 - n;
           h1[R_NTAU] = vn[at(nx, ny - 1)];
           h2[R_NTAU] = vn[at(nx, ny - 2)];
         }

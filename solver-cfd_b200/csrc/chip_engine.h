@@ -23,6 +23,7 @@ struct ChipArgs {
   const int* cases;  // case id per cluster
   int* iters;        // [case * n_steps + step]
   double* err;
+  int corner_role;   // role of the vm buffer whose history gives vm(imax, jmax+1) (see k_chip)
 };
 
 // Shared-memory layout of one CTA, offsets in doubles, the same in every CTA of a cluster: strips of

@@ -1016,7 +1016,7 @@ int run_engine(Batch& b) {
       const bool phys = (cls / 17 - 1) & 1, quick = (cls / 17 - 1) & 2;
       size_t smem = 0;
       for (int q = 0; q < cnt; ++q) smem = std::max(smem, chip_smem(b, order[off + q], K, phys));
-      ChipArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err};
+      ChipArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err, b.engine == 2 ? R_PHYS : R_NTAU};
       e = (b.use_fast ? launch_chip_fast : launch_chip_exact)(a, K, cnt, phys, quick, smem, s);
     } else {
     // staging slot: the largest strip of the size class plus two halo rows on each side
