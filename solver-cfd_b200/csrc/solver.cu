@@ -95,6 +95,7 @@ struct Batch {
   double* d_stage = nullptr;  // staging of field transfers: device, and pinned host for per-routine calls
   double* h_stage = nullptr;
   size_t d_stage_cap = 0, h_stage_cap = 0;  // doubles
+  bool stage_moved = false;   // the stream has changed since d_stage was last used
   int* h_flag = nullptr;  // mapped host word for the host-polled loop
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -246,6 +247,14 @@ bool chip_divisors(const acs_grid& g, const acs_params& p, double phi) {
 }
 
 int push_ctl(Batch& b);
+int flush_ctl(Batch& b);
+
+// Whether a caller is capturing the batch's stream.
+bool capturing(const Batch& b) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(b.stream, &st) != cudaSuccess) cudaGetLastError();
+  return st != cudaStreamCaptureStatusNone;
+}
 
 int field_dims(const CaseDev& d, int family, int* w, int* h) {
   *w = family == 0 ? d.nx + 1 : d.nx;
@@ -255,6 +264,12 @@ int field_dims(const CaseDev& d, int family, int* w, int* h) {
 
 // Staging buffers of at least n doubles, kept with the batch.
 int stage_dev(Batch& b, size_t n) {
+  if (b.stage_moved) {  // transfers on the former stream may still use it; freeing it waits for them
+    if (b.d_stage) cudaFree(b.d_stage);
+    b.d_stage = nullptr;
+    b.d_stage_cap = 0;
+    b.stage_moved = false;
+  }
   if (n <= b.d_stage_cap) return ACS_OK;
   CU(cudaStreamSynchronize(b.stream));
   if (b.d_stage) cudaFree(b.d_stage);
@@ -330,8 +345,32 @@ int prepare_upload(Batch& b, int c, int field, const double* host, FieldLoc* out
   return ACS_OK;
 }
 
+// A field straight from a contiguous host array, without the staging buffer.
+int put(Batch& b, int c, int family, int idx, const double* host) {
+  const CaseDev& d = b.hc[c];
+  int w, h;
+  field_dims(d, family, &w, &h);
+  CU(cudaMemcpy2DAsync(b.buf(c, family, idx), (size_t)d.pitch * 8, host, (size_t)w * 8, (size_t)w * 8, h,
+                       cudaMemcpyHostToDevice, b.stream));
+  return ACS_OK;
+}
+
+// Uploads while a caller captures the batch's stream into a graph: a replay may come when the staging
+// buffer has been replaced, and a capture must not allocate, so every field goes by a copy of its own.
+int capture_uploads(Batch& b, int c, int n, const int* fields, const double* const* host) {
+  int r = flush_ctl(b);
+  for (int q = 0; q < n && !r; ++q) {
+    FieldLoc L;
+    r = prepare_upload(b, c, fields[q], host[q], &L);
+    if (!r && b.ctl_stale) r = push_ctl(b);
+    if (!r) r = put(b, c, L.family, b.role_index(c, L), host[q]);
+  }
+  return r;
+}
+
 // n distinct fields of case c from contiguous host arrays, each applied in the order given.
 int upload_fields(Batch& b, int c, int n, const int* fields, const double* const* host) {
+  if (capturing(b)) return capture_uploads(b, c, n, fields, host);
   MoveList m{};
   for (int q = 0; q < n; ++q) {
     const FieldLoc l = field_loc(fields[q]);
@@ -1142,11 +1181,7 @@ int acs_batch_set_stream(acs_batch* h, void* s) {
   Batch& b = *h->b;
   if (b.gexec) { cudaGraphExecDestroy(b.gexec); b.gexec = nullptr; }
   if (b.graph) { cudaGraphDestroy(b.graph); b.graph = nullptr; }
-  // transfers on the stream so far may still use the staging buffer: it is freed (which waits for them),
-  // and the new stream's first transfer makes its own
-  if (b.d_stage) cudaFree(b.d_stage);
-  b.d_stage = nullptr;
-  b.d_stage_cap = 0;
+  b.stage_moved = true;
   if (s) {
     if (b.own_stream) cudaStreamDestroy(b.stream);
     b.stream = (cudaStream_t)s;
