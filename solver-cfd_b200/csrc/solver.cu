@@ -429,8 +429,24 @@ int push_ctl(Batch& b) {
   CU(cudaMemcpyAsync(b.dk, b.hk.data(), sizeof(CaseCtl) * b.n, cudaMemcpyHostToDevice, b.stream));
   return ACS_OK;
 }
-// before kernels that read the control words outside a run
-int flush_ctl(Batch& b) { return b.ctl_stale ? push_ctl(b) : ACS_OK; }
+// Before kernels that read the control words outside a run.  While a caller captures the stream, the words
+// that earlier uploads changed are copied at once, on a stream of their own: work outside the graph needs
+// them too.
+int flush_ctl(Batch& b) {
+  if (!b.ctl_stale) return ACS_OK;
+  if (!capturing(b)) return push_ctl(b);
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CU(cudaThreadExchangeStreamCaptureMode(&mode));
+  cudaStream_t s = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(b.dk, b.hk.data(), sizeof(CaseCtl) * b.n, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (s) cudaStreamDestroy(s);
+  CU(cudaThreadExchangeStreamCaptureMode(&mode));
+  CU(e);
+  b.ctl_stale = false;
+  return ACS_OK;
+}
 int pull_ctl(Batch& b) {
   CU(cudaMemcpyAsync(b.hk.data(), b.dk, sizeof(CaseCtl) * b.n, cudaMemcpyDeviceToHost, b.stream));
   CU(cudaStreamSynchronize(b.stream));

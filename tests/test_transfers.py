@@ -1,4 +1,5 @@
-"""Field transfers: uploads that a caller captures into a CUDA graph."""
+"""Field transfers: uploads and warm-start hooks that a caller captures into a CUDA graph."""
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +45,34 @@ def test_captured_uploads(gpu, when):
         assert (got["um"] == value).all() and (got["pn"] == 4.0).all()
         b.set_state(0, st)
     b.close()
+
+
+def test_captured_hook_after_an_upload(gpu):
+    """An upload changes the control words (pn gets a buffer of its own again); warm-start features that
+    are captured next leave them right for work outside the graph, before any replay."""
+    import torch
+    prm, mesh, st, itc = _case(gpu)
+    pn = np.asfortranarray(np.random.default_rng(3).uniform(-1, 1, gpu.field_shape("pn", 30, 22)))
+    X = torch.zeros(32 * 32 * 11, device="cuda")
+    sc = torch.zeros(8, device="cuda")
+    outs = []
+    for captured in (False, True):
+        s = torch.cuda.Stream()
+        b = gpu.Batch([prm], [mesh])
+        b.set_stream(s.cuda_stream)
+        b.ws_enable(32, 32)
+        b.set_state(0, st)
+        b.run(1, [itc])
+        b.set_state(0, {"pn": pn})
+        g = torch.cuda.CUDAGraph()
+        if captured:
+            with torch.cuda.graph(g, stream=s):
+                b.ws_features(X.data_ptr(), sc.data_ptr())
+        b.ws_enable(32, 32)
+        b.ws_features(X.data_ptr(), sc.data_ptr())
+        torch.cuda.synchronize()
+        outs.append(X.clone().cpu().numpy())
+        b.close()
+    canvas = outs[0].reshape(32, 32, 11)[:22, :30, 2]
+    assert np.array_equal(canvas, pn.T.astype(np.float32))
+    assert np.array_equal(outs[0], outs[1])
