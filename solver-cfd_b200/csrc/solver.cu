@@ -262,7 +262,10 @@ int field_dims(const CaseDev& d, int family, int* w, int* h) {
   return 0;
 }
 
-// Staging buffers of at least n doubles, kept with the batch.
+// Staging buffers of at least n doubles, kept with the batch, which therefore stay below STAGE_MAX:
+// transfers of more than that go in parts, and a field larger than that by a 2-D copy of its own.  Without
+// the bound the state of a case would need device memory twice.  64 MiB is all 14 fields of 770 x 770 nodes.
+constexpr long long STAGE_MAX = 8ll << 20;
 int stage_dev(Batch& b, size_t n) {
   if (b.stage_moved) {  // transfers on the former stream may still use it; freeing it waits for them
     if (b.d_stage) cudaFree(b.d_stage);
@@ -287,6 +290,12 @@ int stage_host(Batch& b, size_t n) {
   CU(cudaMallocHost(&b.h_stage, n * sizeof(double)));
   b.h_stage_cap = n;
   return ACS_OK;
+}
+
+long long field_size(const Batch& b, int c, int family) {
+  int w, h;
+  field_dims(b.hc[c], family, &w, &h);
+  return (long long)w * h;
 }
 
 // Adds a field of case c to a list of transfers.
@@ -345,13 +354,22 @@ int prepare_upload(Batch& b, int c, int field, const double* host, FieldLoc* out
   return ACS_OK;
 }
 
-// A field straight from a contiguous host array, without the staging buffer.
+// A field straight from or to a contiguous host array, without the staging buffer.
 int put(Batch& b, int c, int family, int idx, const double* host) {
   const CaseDev& d = b.hc[c];
   int w, h;
   field_dims(d, family, &w, &h);
   CU(cudaMemcpy2DAsync(b.buf(c, family, idx), (size_t)d.pitch * 8, host, (size_t)w * 8, (size_t)w * 8, h,
                        cudaMemcpyHostToDevice, b.stream));
+  return ACS_OK;
+}
+
+int get(Batch& b, int c, int family, int idx, double* host) {
+  const CaseDev& d = b.hc[c];
+  int w, h;
+  field_dims(d, family, &w, &h);
+  CU(cudaMemcpy2DAsync(host, (size_t)w * 8, b.buf(c, family, idx), (size_t)d.pitch * 8, (size_t)w * 8, h,
+                       cudaMemcpyDeviceToHost, b.stream));
   return ACS_OK;
 }
 
@@ -368,44 +386,73 @@ int capture_uploads(Batch& b, int c, int n, const int* fields, const double* con
   return r;
 }
 
-// n distinct fields of case c from contiguous host arrays, each applied in the order given.
-int upload_fields(Batch& b, int c, int n, const int* fields, const double* const* host) {
-  if (capturing(b)) return capture_uploads(b, c, n, fields, host);
-  MoveList m{};
-  for (int q = 0; q < n; ++q) {
-    const FieldLoc l = field_loc(fields[q]);
-    if (q && l.role == R_NTAU && l.family >= 0 && l.family != 2 && b.hk[c].ntau_alias) {
-      // n_tau arrays get their own copies now, of what the fields before this one have become
-      int r = upload_fields(b, c, q, fields, host);
-      return r ? r : upload_fields(b, c, n - q, fields + q, host + q);
-    }
-    FieldLoc L;
-    int r = prepare_upload(b, c, fields[q], host[q], &L);
-    if (r) return r;
-    add_move(b, m, c, L.family, b.role_index(c, L));
-  }
+// The transfers listed in m, through the staging buffer; host[q]: the array of m.f[q].
+int move_in(Batch& b, MoveList& m, const double* const* host) {
+  if (!m.n) return ACS_OK;
   int r = stage_dev(b, (size_t)m.total);
   if (r) return r;
-  for (int q = 0; q < n; ++q)
+  for (int q = 0; q < m.n; ++q)
     CU(cudaMemcpyAsync(b.d_stage + m.f[q].off, host[q], sizeof(double) * m.f[q].w * m.f[q].h, cudaMemcpyHostToDevice, b.stream));
   move_to_case(m, b.d_stage, nullptr, CaseCtl{}, b.stream);
   CU(cudaGetLastError());
+  m = MoveList{};
   return ACS_OK;
 }
-
-int download_fields(Batch& b, int c, int n, const int* fields, double* const* host) {
-  MoveList m{};
-  for (int q = 0; q < n; ++q) {
-    FieldLoc L = field_loc(fields[q]);
-    if (L.family < 0) return fail(ACS_E_ARG, "unknown field id");
-    add_move(b, m, c, L.family, b.role_index(c, L));
-  }
+int move_out(Batch& b, MoveList& m, double* const* host) {
+  if (!m.n) return ACS_OK;
   int r = stage_dev(b, (size_t)m.total);
   if (r) return r;
   move_from_case(m, b.d_stage, nullptr, b.stream);
   CU(cudaGetLastError());
-  for (int q = 0; q < n; ++q)
+  for (int q = 0; q < m.n; ++q)
     CU(cudaMemcpyAsync(host[q], b.d_stage + m.f[q].off, sizeof(double) * m.f[q].w * m.f[q].h, cudaMemcpyDeviceToHost, b.stream));
+  m = MoveList{};
+  return ACS_OK;
+}
+
+// n distinct fields of case c from contiguous host arrays, each applied in the order given.
+int upload_fields(Batch& b, int c, int n, const int* fields, const double* const* host) {
+  if (capturing(b)) return capture_uploads(b, c, n, fields, host);
+  MoveList m{};
+  const double* src[MOVE_MAX];
+  for (int q = 0; q < n; ++q) {
+    const FieldLoc l = field_loc(fields[q]);
+    if (l.role == R_NTAU && l.family >= 0 && l.family != 2 && b.hk[c].ntau_alias) {
+      // n_tau arrays get their own copies now, of what the fields before this one have become
+      if (int r = move_in(b, m, src)) return r;
+    }
+    FieldLoc L;
+    int r = prepare_upload(b, c, fields[q], host[q], &L);
+    if (r) return r;
+    const long long size = field_size(b, c, L.family);
+    if (m.total + size > STAGE_MAX && (r = move_in(b, m, src))) return r;
+    if (size > STAGE_MAX) {
+      if ((r = put(b, c, L.family, b.role_index(c, L), host[q]))) return r;
+      continue;
+    }
+    src[m.n] = host[q];
+    add_move(b, m, c, L.family, b.role_index(c, L));
+  }
+  return move_in(b, m, src);
+}
+
+int download_fields(Batch& b, int c, int n, const int* fields, double* const* host) {
+  MoveList m{};
+  double* dst[MOVE_MAX];
+  for (int q = 0; q < n; ++q) {
+    FieldLoc L = field_loc(fields[q]);
+    if (L.family < 0) return fail(ACS_E_ARG, "unknown field id");
+    const long long size = field_size(b, c, L.family);
+    int r = 0;
+    if (m.total + size > STAGE_MAX && (r = move_out(b, m, dst))) return r;
+    if (size > STAGE_MAX) {
+      if ((r = get(b, c, L.family, b.role_index(c, L), host[q]))) return r;
+      continue;
+    }
+    dst[m.n] = host[q];
+    add_move(b, m, c, L.family, b.role_index(c, L));
+  }
+  if (int r = move_out(b, m, dst)) return r;
   CU(cudaStreamSynchronize(b.stream));
   return ACS_OK;
 }
@@ -1109,12 +1156,23 @@ int run_engine(Batch& b) {
 // waits once.
 struct RoutineIO { int family, role; const double* in; double* out; };
 
+long long routine_total(const Batch& b, const RoutineIO* io, int n) {
+  long long t = 4;
+  for (int q = 0; q < n; ++q) t += field_size(b, 0, io[q].family);
+  return t;
+}
+
 int begin_routine(Batch& b, const RoutineIO* io, int n) {
   CaseCtl& k = b.hk[0];
   reset_roles(k);
   k.active = 1;
   k.scalars = 1;
   k.res_u = k.res_v = k.res_p = 0;
+  if (routine_total(b, io, n) > STAGE_MAX) {
+    int r = push_ctl(b);
+    for (int q = 0; q < n && !r; ++q) r = put(b, 0, io[q].family, io[q].role, io[q].in);
+    return r;
+  }
   MoveList m{};
   for (int q = 0; q < n; ++q) add_move(b, m, 0, io[q].family, io[q].role);
   int r = stage_dev(b, (size_t)m.total + 4);
@@ -1129,6 +1187,17 @@ int begin_routine(Batch& b, const RoutineIO* io, int n) {
 }
 
 int end_routine(Batch& b, const RoutineIO* io, int n) {
+  CaseCtl& k = b.hk[0];
+  if (routine_total(b, io, n) > STAGE_MAX) {
+    CU(cudaGetLastError());
+    int r = 0;
+    for (int q = 0; q < n && !r; ++q) r = get(b, 0, io[q].family, io[q].role, io[q].out);
+    if (!r) r = pull_ctl(b);
+    k.active = 0;
+    if (!r) r = push_ctl(b);
+    if (!r) CU(cudaStreamSynchronize(b.stream));
+    return r;
+  }
   MoveList m{};
   for (int q = 0; q < n; ++q) add_move(b, m, 0, io[q].family, io[q].role);
   int r = stage_dev(b, (size_t)m.total + 4);
@@ -1139,7 +1208,6 @@ int end_routine(Batch& b, const RoutineIO* io, int n) {
   CU(cudaMemcpyAsync(b.h_stage, b.d_stage, sizeof(double) * (m.total + 3), cudaMemcpyDeviceToHost, b.stream));
   CU(cudaStreamSynchronize(b.stream));
   for (int q = 0; q < n; ++q) std::memcpy(io[q].out, b.h_stage + m.f[q].off, sizeof(double) * m.f[q].w * m.f[q].h);
-  CaseCtl& k = b.hk[0];
   std::memcpy(&k.res_u, b.h_stage + m.total, 8);
   std::memcpy(&k.res_v, b.h_stage + m.total + 1, 8);
   std::memcpy(&k.res_p, b.h_stage + m.total + 2, 8);

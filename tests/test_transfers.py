@@ -1,4 +1,5 @@
-"""Field transfers: uploads and warm-start hooks that a caller captures into a CUDA graph."""
+"""Field transfers: uploads and warm-start hooks that a caller captures into a CUDA graph, and transfers
+of more than the staging buffer holds (2^23 doubles)."""
 import numpy as np
 import pytest
 
@@ -76,3 +77,45 @@ def test_captured_hook_after_an_upload(gpu):
     canvas = outs[0].reshape(32, 32, 11)[:22, :30, 2]
     assert np.array_equal(canvas, pn.T.astype(np.float32))
     assert np.array_equal(outs[0], outs[1])
+
+
+def _random_state(pkg, nx, ny, names):
+    rng = np.random.default_rng(nx)
+    return {k: np.asfortranarray(rng.uniform(0.5, 1.5, pkg.field_shape(k, nx, ny))) for k in names}
+
+
+# 1999 x 1500: two fields fit in the staging buffer; 3003 x 2900: none does; 2890 x 2902: p fits, vm does not
+@pytest.mark.parametrize("nx,ny", [(1999, 1500), (3003, 2900), (2890, 2902)])
+def test_large_fields_keep_little_memory(gpu, nx, ny):
+    """Fields come back as they were sent, and the device memory that transfers keep is bounded (64 MiB
+    and what the allocator rounds it up to), however large the case."""
+    import torch
+    prm, mesh, st, itc = gpu.configs.channel_case(nx, ny, seed=1)
+    del st
+    names = ("um", "vm", "p", "pn", "T", "um_n_tau")
+    st = _random_state(gpu, nx, ny, names)
+    for make in (gpu.Case, gpu.Batch):
+        b = gpu.Case(prm, mesh) if make is gpu.Case else gpu.Batch([prm], [mesh])
+        args = () if make is gpu.Case else (0,)
+        free = torch.cuda.mem_get_info()[0]
+        b.set_state(*args, st)
+        got = b.get_state(*args, names)
+        assert free - torch.cuda.mem_get_info()[0] <= 80 << 20
+        for k in names:
+            assert np.array_equal(got[k], st[k]), k
+        b.close()
+
+
+def test_large_routine_calls(gpu, orc):
+    """solve_P and solve_U of a case whose fields do not fit in the staging buffer, against the oracle."""
+    nx, ny = 3003, 2900
+    prm, mesh, _, _ = gpu.configs.channel_case(nx, ny, seed=1, scheme=gpu.SCHEME_UPWIND)
+    a = _random_state(gpu, nx, ny, ("um", "um_tau", "vm_tau", "um_n_tau", "vm_n_tau", "p", "pn"))
+    b = {k: v.copy(order="F") for k, v in a.items()}
+    g, o = gpu.Case(prm, mesh), orc.OracleCase(prm, mesh)
+    assert g.solve_P(a["p"], a["um_n_tau"], a["vm_n_tau"], a["pn"]) == o.solve_p(b["p"], b["um_n_tau"], b["vm_n_tau"], b["pn"])
+    assert (g.solve_U(a["um"], None, None, a["um_tau"], a["vm_tau"], a["um_n_tau"], a["pn"])
+            == o.solve_u(b["um"], b["um_tau"], b["vm_tau"], b["pn"], b["um_n_tau"]))
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
+    g.close()
