@@ -119,3 +119,29 @@ def test_large_routine_calls(gpu, orc):
     for k in a:
         assert np.array_equal(a[k], b[k]), k
     g.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(51, 20), (52, 21), (50, 9), (6, 6)])
+@pytest.mark.parametrize("pin", [False, True])
+def test_routes_of_small_fields(gpu, nx, ny, pin):
+    """Fields with and without padding between their rows (um of 51 x 20, vm of 52 x 21 have none), one
+    at a time and together, pageable and pinned, mixed in one call: each comes back as it was sent."""
+    prm, mesh, _, _ = gpu.configs.channel_case(nx, ny, seed=1)
+    st = _random_state(gpu, nx, ny, gpu.FIELDS)
+    if pin:
+        st = {k: (_pinned(a.shape, 0.0)[1], a) for k, a in st.items()}
+        for v, a in st.values():
+            v[:] = a
+        st = {k: v for k, (v, a) in st.items()}
+    b, c = gpu.Batch([prm], [mesh]), gpu.Case(prm, mesh)
+    b.set_state(0, st)
+    c.set_state(st)
+    for got in (b.get_state(0), c.get_state(), {k: b.get_state(0, (k,))[k] for k in st}):
+        for k in st:
+            assert np.array_equal(got[k], st[k]), k
+    out = {k: _pinned(a.shape, -1.0)[1] if pin else np.full_like(a, -1.0) for k, a in st.items()}
+    for k in st:
+        b.get_state(0, (k,), out=out)
+        assert np.array_equal(out[k], st[k]), k
+    b.close()
+    c.close()
