@@ -6,8 +6,9 @@ template <bool PHYS, bool QUICK>
 cudaError_t chip_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int cluster, int nclusters, size_t smem,
                         cudaStream_t s) {
   auto kern = k_chip<PT, PHYS, QUICK>;
+  // attributes belong to the kernel, for every thread of the process: the same values at each launch
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CHIP_MAX_SMEM);
   if (e != cudaSuccess) return e;
   cfg = {};
   cfg.gridDim = dim3(cluster * nclusters);

@@ -49,6 +49,7 @@ struct EngineArgs {
 // stencil into shared-memory slots (cp.async, 16-byte chunks through L2), then computes from
 // them.  One L2 round trip per phase replaces the dependent L2 loads of every node.
 constexpr int STAGE_SLOTS = 7;
+constexpr int STAGE_MAX_BYTES = 220 * 1024;  // dynamic shared memory of the staged engine
 
 // Issues the copy of rows [ra, rb) of a case array into `slot` and returns a pointer that indexes
 // like the global array for those rows.  Rows start on 32-byte boundaries (the pitch is a

@@ -20,8 +20,8 @@ cudaError_t launch_fast_t(const EngineArgs& a, int cluster, int nclusters, cudaS
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   const size_t smem = STG ? (size_t)STAGE_SLOTS * a.stage_elems * sizeof(double) : 0;
-  if (STG) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (STG) {  // the same value at each launch: it belongs to the kernel, for every thread of the process
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGE_MAX_BYTES);
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};

@@ -46,7 +46,6 @@ int fail(int code, const std::string& msg) {
 namespace {
 
 constexpr int kMinN = 6;
-constexpr long long kMaxStageBytes = 220 * 1024;  // dynamic shared memory for the staged engine
 constexpr int kMaxN = 1 << 15;
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -1150,7 +1149,7 @@ int run_engine(Batch& b) {
       slot = std::max(slot, (rows * d.pitch + 1) / 2 * 2);
     }
     const bool stg = b.use_fast && b.staged && b.ctas_per_sm == 1 &&
-                     (long long)STAGE_SLOTS * slot * 8 <= kMaxStageBytes;
+                     (long long)STAGE_SLOTS * slot * 8 <= STAGE_MAX_BYTES;
     EngineArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err, stg ? (int)slot : 0};
     e = b.use_fast ? launch_engine_fast(a, K, cnt, s, b.l1_loads, b.threads, b.ctas_per_sm, stg ? 1 : 0)
                    : launch_engine_exact(a, K, cnt, s);
