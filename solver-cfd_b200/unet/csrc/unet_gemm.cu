@@ -82,7 +82,8 @@ cudaError_t conv_go(const ConvCall& c) {
   a.ty = (a.H + CV_H * MT - 1) / (CV_H * MT);
   const int smem = GATHER ? gather_smem(a.C, a.K, BN) : conv_smem(a.C, BN, MT);
   auto k = k_conv3x3<BN, MT, EPI, GATHER>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // (the same limit at each launch: it belongs to the kernel, for every thread of the process)
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem);
   if (e != cudaSuccess) return e;
   CUtensorMap map;
   if (!weight_map(&map, c.Wt, a.N, a.K, c.ldw, BN)) return cudaErrorInvalidValue;
@@ -133,7 +134,7 @@ template <int BN>
 cudaError_t dx_go(const DxArgs& a, int batch, cudaStream_t s) {
   const int smem = dx_smem(a.N, BN);
   auto k = k_conv_dx<BN>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem);
   if (e != cudaSuccess) return e;
   k<<<dim3((unsigned)(batch * a.ty * a.tx), (unsigned)((a.C + BN - 1) / BN)), TC_THREADS, smem, s>>>(a);
   return cudaGetLastError();

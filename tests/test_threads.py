@@ -26,6 +26,48 @@ def _run(jobs):
     assert not errors, errors
 
 
+@pytest.mark.parametrize("kernel", ["conv3x3", "gather", "dx"])
+def test_network_kernels_of_different_sizes(gpu, kernel):
+    """The same kernel instance for few and for many channels, each thread on its own stream."""
+    import importlib
+    import torch
+    L = importlib.import_module("solver_cfd_b200.unet").kernels()
+    B, H, W, Cout = 1, 16, 16, 32
+
+    def job(Cc, n):
+        s = torch.cuda.Stream()
+        err = torch.zeros(1, dtype=torch.int32, device="cuda")
+        with torch.cuda.stream(s):
+            if kernel == "dx":
+                dz = torch.randn(B * H * W, Cc, device="cuda").to(torch.bfloat16)
+                wt = torch.randn(9 * Cout, Cc, device="cuda").to(torch.bfloat16)
+                y = torch.zeros(B * H * W, Cout, device="cuda")
+            else:
+                x = torch.randn(B * H * W, Cc, device="cuda").to(torch.bfloat16)
+                kp = (9 * Cc + 7) // 8 * 8
+                wt = torch.randn(Cout, kp, device="cuda").to(torch.bfloat16)
+                y = torch.zeros(B * H * W, Cout, device="cuda", dtype=torch.bfloat16)
+        s.synchronize()
+
+        def go():
+            for _ in range(n):
+                if kernel == "dx":
+                    r = L.unet_conv3x3_dx(dz.data_ptr(), wt.data_ptr(), B, H, W, Cout, Cc, y.data_ptr(), err.data_ptr(),
+                                          s.cuda_stream)
+                elif kernel == "gather":
+                    r = L.unet_conv3x3_gather(x.data_ptr(), B, H, W, Cc, wt.data_ptr(), kp, kp, Cout, y.data_ptr(), Cout,
+                                              None, 0, err.data_ptr(), s.cuda_stream)
+                else:
+                    r = L.unet_conv3x3(x.data_ptr(), B, H, W, Cc, wt.data_ptr(), kp, Cout, 2, None, y.data_ptr(), Cout,
+                                       None, 0, err.data_ptr(), s.cuda_stream)
+                assert r == 0, r
+            s.synchronize()
+            assert int(err.item()) == 0
+        return go
+
+    _run([job(3 if kernel == "gather" else 16, 20000), job(11 if kernel == "gather" else 256, 20000)])
+
+
 @pytest.mark.parametrize("arith", [0, 1], ids=["exact", "fast"])
 def test_batches_of_different_sizes(gpu, arith):
     """Batches of small and of larger cases, a few pseudo-iterations per run."""
