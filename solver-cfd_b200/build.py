@@ -44,7 +44,7 @@ SOURCES = {
     "../unet/csrc/unet_ops.cu": [],
 }
 CXX_SOURCES = {"mesh.cpp": ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off"]}
-HEADERS = [os.path.join(ROOT, "include", "unet.h"), "acs_dev.cuh", "kernels.h", "fast.h", "engine.cuh", "engine_api.h", "chip_engine.h", "chip_engine.cuh", "chip_launch.inl", "points_exact.cuh", "points_fast.cuh", "bc_exact.cuh", "warmstart.h", "tile_engine.h", "transfer.h",
+HEADERS = [os.path.join(ROOT, "include", "unet.h"), "acs_dev.cuh", "kernels.h", "fast.h", "engine.cuh", "engine_api.h", "chip_engine.h", "chip_plan.h", "chip_engine.cuh", "chip_launch.inl", "points_exact.cuh", "points_fast.cuh", "bc_exact.cuh", "warmstart.h", "tile_engine.h", "transfer.h",
            "../unet/csrc/gemm_tc.cuh", "../unet/csrc/conv_tc.cuh", "../unet/csrc/conv_grad_tc.cuh"]
 
 

@@ -14,14 +14,13 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <functional>
 #include <string>
 #include <vector>
 
 #include "../../include/acs.h"
 #include "acs_dev.cuh"
 #include "fast.h"
-#include "chip_engine.h"
+#include "chip_plan.h"
 #include "engine_api.h"
 #include "kernels.h"
 #include "tile_engine.h"
@@ -121,11 +120,12 @@ struct Batch {
   int staged = 1;        // FAST engine: stage stencil arrays in shared memory where they fit
   int last_staged = 0;   // the last engine launch used the staged kernel
   std::vector<int> cluster_override;  // per case: CTAs of its cluster (0 = from nodes_per_cta)
-  std::vector<char> chip_ok;          // per case: its constants suit the on-chip engine's arithmetic
+  std::vector<char> chip_ok;          // per case: it has one porosity, no partly porous cells, no artificial
+                                      // divergence damping (b_art) and constants in range (chip_divisors)
   bool user_nodes = false;            // nodes_per_cta was set by the caller
   std::vector<int> chip_k;            // per case: CTAs of its on-chip cluster (0 = cluster engine); built on
                                       // first use, emptied when a launch option changes
-  double chip_us = 0.0;               // modelled time of a pseudo-iteration of all cases on chip (0: not all fit)
+  double chip_us = 0.0;               // ChipPlan::us
   int* d_cases = nullptr;
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> ev;
@@ -1013,67 +1013,19 @@ int cluster_size(const Batch& b, int c) {
   return K;
 }
 
-// Shared memory of one CTA when case c runs on chip in clusters of K (0: it does not fit, or the case
-// has more than one porosity, partly porous cells, artificial
-// divergence damping (b_art) or extreme constants).
-size_t chip_smem(const Batch& b, int c, int K, bool phys) {
+PlanCase plan_case(const Batch& b, int c) {
   const CaseDev& d = b.hc[c];
-  if (!b.chip_ok[c]) return 0;
-  const size_t s = sizeof(double) * (size_t)chip_layout(d.nx, d.ny, d.pitch, K, d.solve_scalars != 0, phys).total;
-  return s <= (size_t)CHIP_MAX_SMEM ? s : 0;
+  const bool user = b.user_nodes || (c < (int)b.cluster_override.size() && b.cluster_override[c] > 0);
+  return {d.nx, d.ny, d.pitch, d.solve_scalars != 0, b.chip_ok[c] != 0, user ? cluster_size(b, c) : 0};
 }
 
-// CTAs of every case's on-chip cluster, 0 where the cluster engine takes the case.  A split that the
-// caller set (ACS_OPT_NODES_PER_CTA, acs_batch_set_cluster_size) is kept.  Otherwise the split with
-// the smallest modelled time of one pseudo-iteration of all cases: a case in K CTAs takes
-// CHIP_T0 + CHIP_T1 * (nodes of its largest strip), and the device runs as many clusters of K at once
-// as its GPCs hold (on a B200 15 of 9 CTAs, 11 of 10, 7 of 11 to 16).
 void chip_plan(Batch& b) {
   if ((int)b.chip_k.size() == b.n) return;
-  b.chip_k.assign(b.n, 0);
-  b.chip_us = 0.0;
-  std::vector<int> kmin(b.n, 0), kmax(b.n, 0), todo;
-  for (int c = 0; c < b.n; ++c) {
-    if (b.user_nodes || (c < (int)b.cluster_override.size() && b.cluster_override[c] > 0)) {
-      const int K = cluster_size(b, c);
-      if (chip_smem(b, c, K, false)) b.chip_k[c] = K;
-      continue;
-    }
-    kmax[c] = std::max(1, std::min(16, (b.hc[c].ny + 1) / 4));
-    for (int K = 1; K <= kmax[c] && !kmin[c]; ++K)
-      if (chip_smem(b, c, K, false)) kmin[c] = K;
-    if (kmin[c]) todo.push_back(c);
-  }
-  if (todo.empty()) return;
-  const double t0 = b.use_fast ? CHIP_T0_FAST : CHIP_T0_EXACT, t1 = b.use_fast ? CHIP_T1_FAST : CHIP_T1_EXACT;
-  double best = 0.0;
-  int best_k = 0;
-  for (int K = 1; K <= 16; ++K) {
-    int kk = 0;
-    std::vector<double> t;
-    for (int c : todo) {
-      const int k = std::min(std::max(K, kmin[c]), kmax[c]);
-      const CaseDev& d = b.hc[c];
-      kk = std::max(kk, k);
-      t.push_back((t0 + t1 * d.nx * ((d.ny + 1 + k - 1) / k)) * (d.solve_scalars ? 1.0 : 0.6));
-    }
-    const int slots = std::max(1, (b.use_fast ? chip_resident_fast : chip_resident_exact)(kk));
-    // longest first onto the slot that is free first
-    std::sort(t.begin(), t.end(), std::greater<double>());
-    std::vector<double> busy(std::min((size_t)slots, t.size()), 0.0);
-    for (double x : t) {
-      std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
-      busy.back() += x;
-      std::push_heap(busy.begin(), busy.end(), std::greater<double>());
-    }
-    const double end = *std::max_element(busy.begin(), busy.end());
-    if (!best_k || end < best) {
-      best = end;
-      best_k = K;
-    }
-  }
-  for (int c : todo) b.chip_k[c] = std::min(std::max(best_k, kmin[c]), kmax[c]);
-  if ((int)todo.size() == b.n) b.chip_us = best;
+  std::vector<PlanCase> cases;
+  for (int c = 0; c < b.n; ++c) cases.push_back(plan_case(b, c));
+  ChipPlan p = plan_chip(cases, b.use_fast, b.use_fast ? chip_resident_fast : chip_resident_exact);
+  b.chip_k = std::move(p.k);
+  b.chip_us = p.us;
 }
 
 // Whether a batch on the tile engine is faster on chip: the tile engine's seven launches of a
@@ -1098,7 +1050,7 @@ int run_engine(Batch& b) {
   std::vector<std::vector<int>> groups(kClasses);
   for (int c = 0; c < b.n; ++c) {
     const int K = b.chip_k[c];
-    const int kind = 1 + (K && chip_smem(b, c, K, true) ? 1 : 0) + (b.hc[c].scheme == 0 ? 2 : 0);
+    const int kind = 1 + (K && chip_bytes(plan_case(b, c), K, true) ? 1 : 0) + (b.hc[c].scheme == 0 ? 2 : 0);
     groups[!K ? cluster_size(b, c) : 17 * kind + K].push_back(c);
   }
   if (!b.d_cases) CU(cudaMalloc(&b.d_cases, sizeof(int) * b.n));
@@ -1137,7 +1089,7 @@ int run_engine(Batch& b) {
     if (cls >= 17) {
       const bool phys = (cls / 17 - 1) & 1, quick = (cls / 17 - 1) & 2;
       size_t smem = 0;
-      for (int q = 0; q < cnt; ++q) smem = std::max(smem, chip_smem(b, order[off + q], K, phys));
+      for (int q = 0; q < cnt; ++q) smem = std::max(smem, chip_bytes(plan_case(b, order[off + q]), K, phys));
       ChipArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err, b.engine == 2 ? R_PHYS : R_NTAU};
       e = (b.use_fast ? launch_chip_fast : launch_chip_exact)(a, K, cnt, phys, quick, smem, s);
     } else {
