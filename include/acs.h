@@ -237,7 +237,8 @@ enum acs_option {
                                    the environment variable ACS_NO_CONDITIONAL_GRAPH set, engines 1
                                    and 2 loop from the host instead (one graph launch per
                                    pseudo-iteration), which profilers can look inside */
-  ACS_OPT_NODES_PER_CTA = 2, /* engine: target nodes per CTA when sizing a case's cluster */
+  ACS_OPT_NODES_PER_CTA = 2, /* engine: target nodes per CTA when sizing a case's cluster (more CTAs
+                                where a case only fits on chip in more) */
   ACS_OPT_L1_LOADS = 3,      /* FAST engine: 1 (default) reads cluster-written arrays through L1 */
   ACS_OPT_THREADS = 4,       /* FAST engine: threads per CTA, 256 or 512 (default) */
   ACS_OPT_CTAS_PER_SM = 5,   /* FAST engine, 256 threads: 2 caps registers so two CTAs share an SM */
@@ -254,7 +255,8 @@ int acs_batch_set_option(acs_batch* b, int option, long long value);
  * case_id's cluster, overriding ACS_OPT_NODES_PER_CTA for that case; 0 restores the default.
  * A batched step lasts as long as its slowest case, so a caller that knows which cases need the
  * most pseudo-iterations (e.g. from the previous step) can give them more CTAs.  Still capped at
- * (jmax+1)/4 (strips of at least 4 rows).  Results do not depend on it. */
+ * (jmax+1)/4 (strips of at least 4 rows), and a case that runs on chip gets the next larger number that
+ * it fits in.  Results do not depend on it. */
 int acs_batch_set_cluster_size(acs_batch* b, int case_id, int ctas);
 /* The pseudo-time residual tolerance of case case_id for the following steps: the `eps` of the
  * exit test `error < eps` (main.f90:142; read from input/iterations.dat), initially the

@@ -16,8 +16,7 @@ struct PlanCase {
 };
 struct ChipPlan {
   std::vector<int> k;  // CTAs of every case's on-chip cluster, 0 where the cluster engine takes the case
-  double us = 0.0;     // modelled time of a pseudo-iteration of all cases on chip (0: not all fit, or a
-                       // caller's split)
+  double us = 0.0;     // modelled time of a pseudo-iteration of all cases on chip (0: not all fit)
 };
 
 // Shared memory of one CTA when a case runs on chip in clusters of K (0: it does not fit).
@@ -27,11 +26,15 @@ inline size_t chip_bytes(const PlanCase& c, int K, bool phys) {
   return s <= (size_t)CHIP_MAX_SMEM ? s : 0;
 }
 
-// A split that the caller asks for is kept.  Otherwise the split with the smallest modelled time of one
-// pseudo-iteration of all cases: a case in K CTAs takes CHIP_T0 + CHIP_T1 * (nodes of its largest strip),
-// and the device runs as many clusters of K at once as its GPCs hold (on a B200 15 of 9 CTAs, 11 of 10, 7 of
-// 11 to 16).  resident(K): that number; sizes that the device cannot hold at all (0: fewer SMs, or a share
-// of the device) are left out, and a case that only fits in such a size goes to the cluster engine.
+// Whether a case runs on chip depends on the case and the device only, so a split that the caller asks for
+// changes no result: it is the size asked for where the case fits in that, else the next larger one that it
+// fits in, else its largest.  (Left to the cluster engine, a 102 x 102 FAST case asked into 4 CTAs had other
+// roundings and about four times the time per pseudo-iteration.)  The other cases get the split with the
+// smallest modelled time of one pseudo-iteration of all cases: a case in K CTAs takes
+// CHIP_T0 + CHIP_T1 * (nodes of its largest strip), and the device runs as many clusters of K at once as its
+// GPCs hold (on a B200 15 of 9 CTAs, 11 of 10, 7 of 11 to 16).  resident(K): that number; sizes that the
+// device cannot hold at all (0: fewer SMs, or a share of the device) are left out, and a case that only fits
+// in such a size goes to the cluster engine.
 inline ChipPlan plan_chip(const std::vector<PlanCase>& cases, bool fast, const std::function<int(int)>& resident) {
   const int n = (int)cases.size();
   ChipPlan p;
@@ -44,26 +47,24 @@ inline ChipPlan plan_chip(const std::vector<PlanCase>& cases, bool fast, const s
   };
   std::vector<std::vector<int>> sizes(n);  // cluster sizes that take the case, ascending
   std::vector<int> todo;
+  bool free_split = false;  // some case's split is the plan's own
   for (int c = 0; c < n; ++c) {
-    if (cases[c].want) {
-      if (chip_bytes(cases[c], cases[c].want, false) && res(cases[c].want) > 0) p.k[c] = cases[c].want;
-      continue;
-    }
     const int kmax = std::max(1, std::min(16, (cases[c].ny + 1) / 4));
     for (int K = 1; K <= kmax; ++K)
       if (chip_bytes(cases[c], K, false) && res(K) > 0) sizes[c].push_back(K);
     if (!sizes[c].empty()) todo.push_back(c);
+    free_split |= !sizes[c].empty() && !cases[c].want;
   }
   if (todo.empty()) return p;
-  // the smallest size of case c that is at least K, else its largest
+  // the smallest size of case c that is at least what is asked for (by the caller, else K), else its largest
   auto at_least = [&](int c, int K) {
-    auto it = std::lower_bound(sizes[c].begin(), sizes[c].end(), K);
+    auto it = std::lower_bound(sizes[c].begin(), sizes[c].end(), cases[c].want ? cases[c].want : K);
     return it == sizes[c].end() ? sizes[c].back() : *it;
   };
   const double t0 = fast ? CHIP_T0_FAST : CHIP_T0_EXACT, t1 = fast ? CHIP_T1_FAST : CHIP_T1_EXACT;
   double best = 0.0;
   int best_k = 0;
-  for (int K = 1; K <= 16; ++K) {
+  for (int K = 1; K <= (free_split ? 16 : 1); ++K) {
     int kk = 0;
     std::vector<double> t;
     for (int c : todo) {

@@ -59,4 +59,17 @@ def test_sizes_that_the_device_cannot_hold_are_left_out(plan):
     for most in range(1, 17):
         plan([small, full, (30, 22, 0, 0), (40, 9, 1, 0)], most=most)
     assert plan([small, (30, 22, 0, 0)], most=0) == ([0, 0], 0.0)
-    assert plan([(51, 51, 1, 9)], most=8)[0] == [0]
+    assert plan([(51, 51, 1, 9)], most=8)[0] == [8]
+
+
+def test_a_caller_s_split_does_not_move_a_case_off_the_chip(plan):
+    """The size asked for where the case fits in it, else the next larger one that it fits in."""
+    assert [plan([(51, 51, 1, K)])[0][0] for K in (4, 9, 12)] == [4, 9, 12]
+    least = next(K for K in range(1, 17) if plan([(102, 102, 1, K)])[0] == [K])
+    assert least > 4
+    for K in range(1, 17):
+        assert plan([(102, 102, 1, K)])[0] == [max(K, least)]
+        assert plan([(153, 153, 1, K)])[0] == [16]
+        assert plan([(300, 300, 1, K)])[0] == [0]          # too large for any cluster
+    k, us = plan([(51, 51, 1, 4), (51, 51, 1, 0)])
+    assert k[0] == 4 and k[1] > 0 and us > 0
