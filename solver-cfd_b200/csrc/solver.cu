@@ -794,7 +794,7 @@ LoopEnd loop_end(Batch& b, int mode) {
   return e;
 }
 
-void launch_control(Batch& b, const LoopEnd& end) {
+cudaError_t launch_control(Batch& b, const LoopEnd& end) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(b.n);
   cfg.blockDim = dim3(256);
@@ -804,21 +804,23 @@ void launch_control(Batch& b, const LoopEnd& end) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = b.engine == 2 && b.overlap ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k_control, (const CaseDev*)b.dc, b.dk, b.d_iters, b.d_err, b.d_nactive, end);
   b.launches += 1;
+  return cudaLaunchKernelEx(&cfg, k_control, (const CaseDev*)b.dc, b.dk, b.d_iters, b.d_err, b.d_nactive, end);
 }
 
-// one pseudo-iteration of the tile engine: U/V stages 1-3, P + T/C, control
-void te_iteration(Batch& b, const LoopEnd& end) {
-  for (int s = 1; s <= 3; ++s)
-    te_launch_uv(s, b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.overlap && s > 1, b.stream);
-  te_launch_ptc(b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.overlap, b.stream);
+// One pseudo-iteration of the tile engine: U/V stages 1-3, P + T/C, control.  Returns the first launch error,
+// as loop_body does: a loop body without one of its kernels must not run (k_control ends the loop).
+cudaError_t te_iteration(Batch& b, const LoopEnd& end) {
+  cudaError_t e = cudaSuccess;
+  for (int s = 1; s <= 3 && e == cudaSuccess; ++s)
+    e = te_launch_uv(s, b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.overlap && s > 1, b.stream);
+  if (e == cudaSuccess) e = te_launch_ptc(b.dc, b.dk, b.d_tetiles, b.n_tetiles, b.d_temaps, b.d_te_err, b.overlap, b.stream);
   b.launches += 4;
-  launch_control(b, end);
+  return e == cudaSuccess ? launch_control(b, end) : e;
 }
 
 // one pseudo-iteration (main.f90:122-150) for every active case
-void seq_iteration(Batch& b, const LoopEnd& end) {
+cudaError_t seq_iteration(Batch& b, const LoopEnd& end) {
   seq_u(b);
   seq_v(b);
   seq_p(b);
@@ -826,7 +828,15 @@ void seq_iteration(Batch& b, const LoopEnd& end) {
     seq_s(b, false);
     seq_s(b, true);
   }
-  launch_control(b, end);
+  return launch_control(b, end);
+}
+
+// The body of the pseudo-time loop, captured on the batch's stream.
+cudaError_t loop_body(Batch& b, const LoopEnd& end) {
+  cudaGetLastError();
+  const cudaError_t e = b.engine == 2 ? te_iteration(b, end) : seq_iteration(b, end);
+  const cudaError_t any = cudaGetLastError();  // of the launches whose status is not returned
+  return e != cudaSuccess ? e : any;
 }
 
 long long max_total_iterations(const Batch& b, int n_steps) {
@@ -862,10 +872,10 @@ int build_graph(Batch& b, int n_steps) {
         LoopEnd end = loop_end(b, LOOP_COND);
         end.handle = h;
         end.max_iters = max_total_iterations(b, n_steps);
-        if (b.engine == 2) te_iteration(b, end);
-        else seq_iteration(b, end);
+        const cudaError_t launched = loop_body(b, end);
         b.body_kernels = b.launches - l0;
         e = cudaStreamEndCapture(b.stream, &body);
+        if (launched != cudaSuccess) e = launched;
       }
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&b.gexec, g, 0);
@@ -892,10 +902,13 @@ int build_graph(Batch& b, int n_steps) {
   const long long l0 = b.launches;
   LoopEnd end = loop_end(b, LOOP_FLAG);
   end.host_flag = d_flag;
-  if (b.engine == 2) te_iteration(b, end);
-  else seq_iteration(b, end);
+  const cudaError_t launched = loop_body(b, end);
   b.body_kernels = b.launches - l0;
   CU(cudaStreamEndCapture(b.stream, &g));
+  if (launched != cudaSuccess) {
+    cudaGraphDestroy(g);
+    return fail(ACS_E_CUDA, std::string("loop body: ") + cudaGetErrorString(launched));
+  }
   CU(cudaGraphInstantiate(&b.gexec, g, 0));
   b.graph = g;
   b.launches = saved;

@@ -692,7 +692,7 @@ cudaError_t te_prepare() {
 
 namespace {
 template <class K, class... A>
-void te_launch(K kern, int grid, size_t smem, bool overlap, cudaStream_t s, A... args) {
+cudaError_t te_launch(K kern, int grid, size_t smem, bool overlap, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(TE_THREADS);
@@ -703,20 +703,20 @@ void te_launch(K kern, int grid, size_t smem, bool overlap, cudaStream_t s, A...
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kern, args...);
+  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 }  // namespace
 
-void te_launch_uv(int stage, const CaseDev* cs, CaseCtl* ctl, const Tile* tiles, int ntiles, const TeMaps* maps,
+cudaError_t te_launch_uv(int stage, const CaseDev* cs, CaseCtl* ctl, const Tile* tiles, int ntiles, const TeMaps* maps,
                   int* err, bool overlap, cudaStream_t s) {
-  if (stage == 1) te_launch(k_te_uv<1>, ntiles, smem_uv<1>(), overlap, s, cs, ctl, tiles, maps, err);
-  else if (stage == 2) te_launch(k_te_uv<2>, ntiles, smem_uv<2>(), overlap, s, cs, ctl, tiles, maps, err);
-  else te_launch(k_te_uv<3>, ntiles, smem_uv<3>(), overlap, s, cs, ctl, tiles, maps, err);
+  if (stage == 1) return te_launch(k_te_uv<1>, ntiles, smem_uv<1>(), overlap, s, cs, ctl, tiles, maps, err);
+  if (stage == 2) return te_launch(k_te_uv<2>, ntiles, smem_uv<2>(), overlap, s, cs, ctl, tiles, maps, err);
+  return te_launch(k_te_uv<3>, ntiles, smem_uv<3>(), overlap, s, cs, ctl, tiles, maps, err);
 }
 
-void te_launch_ptc(const CaseDev* cs, CaseCtl* ctl, const Tile* tiles, int ntiles, const TeMaps* maps, int* err,
+cudaError_t te_launch_ptc(const CaseDev* cs, CaseCtl* ctl, const Tile* tiles, int ntiles, const TeMaps* maps, int* err,
                    bool overlap, cudaStream_t s) {
-  te_launch(k_te_ptc, ntiles, SMEM_PTC2, overlap, s, cs, ctl, tiles, maps, err);
+  return te_launch(k_te_ptc, ntiles, SMEM_PTC2, overlap, s, cs, ctl, tiles, maps, err);
 }
 
 }  // namespace acs

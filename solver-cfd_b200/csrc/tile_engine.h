@@ -47,10 +47,10 @@ int te_encode_maps(const std::vector<CaseDev>& cases, TeMaps* maps);
 // Launches of one pseudo-iteration (without the control kernel).  err: device word set to a
 // nonzero code when a TMA wait times out.
 // overlap: the launch may begin while the kernel before it in the stream drains (programmatic dependent launch).
-void te_launch_uv(int stage, const CaseDev* cs, CaseCtl* ctl, const Tile* tiles, int ntiles, const TeMaps* maps,
-                  int* err, bool overlap, cudaStream_t s);
-void te_launch_ptc(const CaseDev* cs, CaseCtl* ctl, const Tile* tiles, int ntiles, const TeMaps* maps, int* err,
-                   bool overlap, cudaStream_t s);
+cudaError_t te_launch_uv(int stage, const CaseDev* cs, CaseCtl* ctl, const Tile* tiles, int ntiles, const TeMaps* maps,
+                         int* err, bool overlap, cudaStream_t s);
+cudaError_t te_launch_ptc(const CaseDev* cs, CaseCtl* ctl, const Tile* tiles, int ntiles, const TeMaps* maps, int* err,
+                          bool overlap, cudaStream_t s);
 // One-time kernel attributes (dynamic shared memory sizes); returns the first error.
 cudaError_t te_prepare();
 
