@@ -232,8 +232,8 @@ enum acs_option {
                                    memory by TMA, four stage kernels per pseudo-iteration in a CUDA graph
                                    with a device WHILE node -- the fastest for many cases; a batch
                                    whose cases all fit on chip and iterate faster there (a few
-                                   cases) runs as with 0.  Setting
-                                   it builds the tile table and tensor maps (device memory).  With
+                                   cases) runs as with 0 (ACS_OPT_ON_CHIP = 1 keeps the tile
+                                   kernels).  Setting it builds the tile table and tensor maps (device memory).  With
                                    the environment variable ACS_NO_CONDITIONAL_GRAPH set, engines 1
                                    and 2 loop from the host instead (one graph launch per
                                    pseudo-iteration), which profilers can look inside */
@@ -245,11 +245,22 @@ enum acs_option {
   ACS_OPT_STAGED = 6,        /* FAST engine: 1 (default) copies each phase's stencil arrays (the
                                 CTA's rows plus two halo rows) into shared memory first, where
                                 they fit in 220 KB; 0 reads them from L1/L2 */
-  ACS_OPT_EXTRAP_ORDER = 7   /* warm start: the extrapolated candidate of acs_batch_set_start is
+  ACS_OPT_EXTRAP_ORDER = 7,  /* warm start: the extrapolated candidate of acs_batch_set_start is
                                 x + inc (1, default) or x + (2 inc - inc_prev), the quadratic
                                 through the last three step starts (2; linear until three
                                 acs_batch_ws_features calls have given two increments) */
+  ACS_OPT_ON_CHIP = 8        /* engines 0 and 2: 0 (default) runs cases on chip as described above,
+                                1 never does */
 };
+/* EXACT results are the same bits on every engine.  FAST results agree to 1e-10 between the cluster
+ * engine, the graph engine, the tile engine and the on-chip kernels, not bit for bit; with engine 0
+ * the kernel depends on the case alone, with engine 2 on the whole batch, unless ACS_OPT_ON_CHIP is 1.
+ * Options 3 to 6 only concern the cluster engine, i.e. cases that do not run on chip.
+ * acs_batch_engines_used / acs_engines_used: which kernels the last run used, a sum of enum acs_used
+ * (0 before the first run). */
+enum acs_used { ACS_USED_CLUSTER = 1, ACS_USED_GRAPH = 2, ACS_USED_TILE = 4, ACS_USED_CHIP = 8 };
+int acs_batch_engines_used(acs_batch* b, int* used);
+int acs_engines_used(acs_handle* h, int* used);
 int acs_batch_set_option(acs_batch* b, int option, long long value);
 /* Persistent cluster engine (no reference counterpart): the number of CTAs (1..16) of case
  * case_id's cluster, overriding ACS_OPT_NODES_PER_CTA for that case; 0 restores the default.

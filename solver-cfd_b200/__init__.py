@@ -47,14 +47,15 @@ EXPORTED = (
     "acs_batch_set_option", "acs_set_option", "acs_solve_u_static",
     "acs_batch_ws_enable", "acs_batch_ws_features", "acs_batch_ws_target", "acs_batch_set_start",
     "acs_batch_set_cluster_size", "acs_batch_set_tolerance", "acs_batch_cell_fields", "acs_cell_fields",
-    "acs_mesh_channel_device",
+    "acs_mesh_channel_device", "acs_batch_engines_used", "acs_engines_used",
 )
 WS_IN, WS_OUT = 11, 8
 POLICY_BEST, POLICY_PREDICTED, POLICY_PLAIN = 0, 1, 2
 START_PLAIN, START_EXTRAP, START_LEARNED = 0, 1, 2
 OPT_ENGINE, OPT_NODES_PER_CTA, OPT_L1_LOADS, OPT_THREADS, OPT_CTAS_PER_SM, OPT_STAGED = 1, 2, 3, 4, 5, 6
-OPT_EXTRAP_ORDER = 7
+OPT_EXTRAP_ORDER, OPT_ON_CHIP = 7, 8
 ENGINE_CLUSTER, ENGINE_GRAPH, ENGINE_TILE = 0, 1, 2
+USED_CLUSTER, USED_GRAPH, USED_TILE, USED_CHIP = 1, 2, 4, 8
 
 
 class AcsError(RuntimeError):
@@ -132,6 +133,8 @@ def _declare(L):
     L.acs_batch_run.argtypes = [V, C.c_int, _I, _I, _D, _I]
     L.acs_batch_launch_count.argtypes = [V, C.POINTER(C.c_longlong)]
     L.acs_launch_count.argtypes = [V, C.POINTER(C.c_longlong)]
+    L.acs_batch_engines_used.argtypes = [V, _I]
+    L.acs_engines_used.argtypes = [V, _I]
     L.acs_batch_time_kernel.argtypes = [V, C.c_int, C.c_int, _D, C.POINTER(C.c_longlong)]
     L.acs_batch_set_option.argtypes = [V, C.c_int, C.c_longlong]
     L.acs_set_option.argtypes = [V, C.c_int, C.c_longlong]
@@ -356,6 +359,12 @@ class Case:
         _check(lib().acs_launch_count(self.h, C.byref(n)), "acs_launch_count")
         return n.value
 
+    def engines_used(self) -> int:
+        """Which kernels the last run used: a sum of USED_*."""
+        n = C.c_int(0)
+        _check(lib().acs_engines_used(self.h, C.byref(n)), "acs_engines_used")
+        return n.value
+
     def cell_fields(self):
         """comp_mean on the device: cell-centred (u, v) and the velocity magnitude."""
         out = [np.zeros((self.nx, self.ny), order="F") for _ in range(3)]
@@ -433,6 +442,12 @@ class Batch:
     def launch_count(self) -> int:
         n = C.c_longlong(0)
         _check(lib().acs_batch_launch_count(self.h, C.byref(n)), "acs_batch_launch_count")
+        return n.value
+
+    def engines_used(self) -> int:
+        """Which kernels the last run used: a sum of USED_*."""
+        n = C.c_int(0)
+        _check(lib().acs_batch_engines_used(self.h, C.byref(n)), "acs_batch_engines_used")
         return n.value
 
     def cell_fields(self, c: int):

@@ -118,7 +118,8 @@ struct Batch {
   int threads = 512;     // FAST engine: threads per CTA (256 or 512)
   int ctas_per_sm = 1;   // FAST engine with 256 threads: 1 or 2 resident CTAs per SM
   int staged = 1;        // FAST engine: stage stencil arrays in shared memory where they fit
-  int last_staged = 0;   // the last engine launch used the staged kernel
+  bool on_chip = true;   // ACS_OPT_ON_CHIP
+  int used = 0;          // enum acs_used of the last run
   std::vector<int> cluster_override;  // per case: CTAs of its cluster (0 = from nodes_per_cta)
   std::vector<char> chip_ok;          // per case: it has one porosity, no partly porous cells, no artificial
                                       // divergence damping (b_art) and constants in range (chip_divisors)
@@ -951,10 +952,12 @@ int run_batch(Batch& b, int n_steps, int* itc, int* iters, double* err, int* sta
   r = push_ctl(b);
   if (r) return r;
   CU(cudaMemsetAsync(b.d_nactive, 0, 256, b.stream));
+  b.used = 0;
   if (b.engine == 0 || (b.engine == 2 && chip_beats_tiles(b))) {
     r = run_engine(b);
     if (r) return r;
   } else {
+    b.used = b.engine == 2 ? ACS_USED_TILE : ACS_USED_GRAPH;
     r = run_graph(b, n_steps);
     if (r) return r;
   }
@@ -1029,7 +1032,7 @@ int cluster_size(const Batch& b, int c) {
 PlanCase plan_case(const Batch& b, int c) {
   const CaseDev& d = b.hc[c];
   const bool user = b.user_nodes || (c < (int)b.cluster_override.size() && b.cluster_override[c] > 0);
-  return {d.nx, d.ny, d.pitch, d.solve_scalars != 0, b.chip_ok[c] != 0, user ? cluster_size(b, c) : 0};
+  return {d.nx, d.ny, d.pitch, d.solve_scalars != 0, b.on_chip && b.chip_ok[c], user ? cluster_size(b, c) : 0};
 }
 
 void chip_plan(Batch& b) {
@@ -1118,13 +1121,13 @@ int run_engine(Batch& b) {
     EngineArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err, stg ? (int)slot : 0};
     e = b.use_fast ? launch_engine_fast(a, K, cnt, s, b.l1_loads, b.threads, b.ctas_per_sm, stg ? 1 : 0)
                    : launch_engine_exact(a, K, cnt, s);
-    b.last_staged = stg ? 1 : 0;
     }
     if (e != cudaSuccess) {
       cudaEventDestroy(fork);
       return fail(ACS_E_CUDA, std::string("engine launch (cluster ") + std::to_string(K) + "): " + cudaGetErrorString(e));
     }
     b.launches += 1;
+    b.used |= cls >= 17 ? ACS_USED_CHIP : ACS_USED_CLUSTER;
     if (g) {
       CU(cudaEventRecord(b.ev[g], s));
       CU(cudaStreamWaitEvent(b.stream, b.ev[g], 0));
@@ -1523,6 +1526,11 @@ int acs_batch_set_option(acs_batch* h, int option, long long value) {
     case ACS_OPT_STAGED:
       b.staged = value ? 1 : 0;
       return ACS_OK;
+    case ACS_OPT_ON_CHIP:
+      if (value != 0 && value != 1) return acs::fail(ACS_E_ARG, "on-chip option must be 0 or 1");
+      b.on_chip = value == 0;
+      b.chip_k.clear();
+      return ACS_OK;
     case ACS_OPT_EXTRAP_ORDER:
       if (value != 1 && value != 2) return acs::fail(ACS_E_ARG, "extrapolation order must be 1 or 2");
       b.ws_order = (int)value;
@@ -1540,6 +1548,12 @@ int acs_set_option(acs_handle* h, int option, long long value) {
 int acs_batch_launch_count(acs_batch* h, long long* n) {
   if (!h || !n) return acs::fail(ACS_E_ARG, "null");
   *n = h->b->launches;
+  return ACS_OK;
+}
+
+int acs_batch_engines_used(acs_batch* h, int* used) {
+  if (!h || !used) return acs::fail(ACS_E_ARG, "null");
+  *used = h->b->used;
   return ACS_OK;
 }
 
@@ -1592,6 +1606,12 @@ int acs_physical_steps(acs_handle* h, int n_steps, int* itc, int* iters, double*
 int acs_launch_count(acs_handle* h, long long* n) {
   if (!h || !n) return acs::fail(ACS_E_ARG, "null");
   *n = h->b->launches;
+  return ACS_OK;
+}
+
+int acs_engines_used(acs_handle* h, int* used) {
+  if (!h || !used) return acs::fail(ACS_E_ARG, "null");
+  *used = h->b->used;
   return ACS_OK;
 }
 

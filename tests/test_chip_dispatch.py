@@ -29,3 +29,42 @@ def test_fast_results_do_not_depend_on_the_split(gpu):
             assert np.array_equal(it, ref[0]) and np.array_equal(er, ref[1]), K
             for k in out:
                 assert np.array_equal(out[k], ref[2][k]), (K, k)
+
+
+def test_the_choice_of_kernels(gpu):
+    """What the library chooses by itself, and with ACS_OPT_ON_CHIP = 1."""
+    small = _item(gpu, 30, 22, itc_max=4, arith=gpu.ARITH_FAST)
+    art = gpu.configs.reference_case(12, itc_max=4, b_art=0.3)[:4]
+    large = _item(gpu, 300, 300, itc_max=4, arith=gpu.ARITH_FAST)
+
+    def used(item, n, engine, on_chip):
+        b = gpu.Batch([item[0]] * n, [item[1]] * n)
+        assert b.engines_used() == 0
+        b.set_option(gpu.OPT_ENGINE, engine)
+        b.set_option(gpu.OPT_ON_CHIP, on_chip)
+        for c in range(n):
+            b.set_state(c, item[2])
+        b.run(1, item[3])
+        r = b.engines_used()
+        b.set_option(gpu.OPT_ON_CHIP, 1 - on_chip)  # takes effect with the next run
+        b.run(1, item[3])
+        assert r in (gpu.USED_CLUSTER, gpu.USED_GRAPH, gpu.USED_TILE, gpu.USED_CHIP)
+        b.close()
+        return r
+
+    assert used(small, 3, gpu.ENGINE_CLUSTER, 0) == gpu.USED_CHIP
+    assert used(small, 3, gpu.ENGINE_CLUSTER, 1) == gpu.USED_CLUSTER
+    assert used(small, 3, gpu.ENGINE_TILE, 0) == gpu.USED_CHIP
+    assert used(small, 3, gpu.ENGINE_TILE, 1) == gpu.USED_TILE
+    assert used(small, 3, gpu.ENGINE_GRAPH, 0) == gpu.USED_GRAPH
+    assert used(art, 1, gpu.ENGINE_CLUSTER, 0) == gpu.USED_CLUSTER
+    assert used(large, 1, gpu.ENGINE_CLUSTER, 0) == gpu.USED_CLUSTER
+    assert used(large, 1, gpu.ENGINE_TILE, 0) == gpu.USED_TILE
+    c = gpu.Case(small[0], small[1])
+    c.set_state(small[2])
+    c.physical_steps(1, small[3])
+    assert c.engines_used() == gpu.USED_CHIP
+    for bad in (-1, 2):
+        with pytest.raises(gpu.AcsError):
+            c.set_option(gpu.OPT_ON_CHIP, bad)
+    c.close()
