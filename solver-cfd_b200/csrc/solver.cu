@@ -1050,7 +1050,6 @@ void chip_plan(Batch& b) {
 // iterate side by side in 15 to 30 us (3 cases of 101 x 147: 51 us against 19).  Only a clear advantage
 // of the modelled times counts.
 bool chip_beats_tiles(Batch& b) {
-  if (getenv("ACS_NO_CONDITIONAL_GRAPH")) return false;  // a profiler wants the tile kernels
   chip_plan(b);
   double nodes = 0.0;
   for (int c = 0; c < b.n; ++c) nodes += (double)b.hc[c].nx * b.hc[c].ny;

@@ -68,3 +68,24 @@ def test_the_choice_of_kernels(gpu):
         with pytest.raises(gpu.AcsError):
             c.set_option(gpu.OPT_ON_CHIP, bad)
     c.close()
+
+
+@pytest.mark.parametrize("n,nx,ny,used", [(3, 40, 30, "USED_CHIP"), (1, 40, 30, "USED_CHIP"), (2, 300, 300, "USED_TILE")])
+def test_loop_kind_does_not_choose_kernels(gpu, monkeypatch, n, nx, ny, used):
+    """ACS_NO_CONDITIONAL_GRAPH sets how the loop of the graph and tile engines is driven; the kernels of a
+    batch, and so its bits, stay."""
+    item = _item(gpu, nx, ny, itc_max=12, arith=gpu.ARITH_FAST)
+    outs = []
+    for env in (False, True):
+        if env:
+            monkeypatch.setenv("ACS_NO_CONDITIONAL_GRAPH", "1")
+        b = gpu.Batch([item[0]] * n, [item[1]] * n)
+        b.set_option(gpu.OPT_ENGINE, gpu.ENGINE_TILE)
+        for c in range(n):
+            b.set_state(c, item[2])
+        b.run(1, item[3])
+        assert b.engines_used() == getattr(gpu, used)
+        outs.append(b.get_state(n - 1))
+        b.close()
+    for k in outs[0]:
+        assert np.array_equal(outs[0][k], outs[1][k]), k
