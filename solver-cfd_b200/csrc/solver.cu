@@ -1044,11 +1044,13 @@ void chip_plan(Batch& b) {
   b.chip_us = p.us;
 }
 
-// Whether a batch on the tile engine is faster on chip: the tile engine's seven launches of a
-// pseudo-iteration take at least 50 us, and 0.165 us per 1000 nodes once they fill the device (measured:
-// 45,000 nodes 51 us, 0.52 million 105, 1.5 million 273, 4.1 million 770), while a few cases in clusters
-// iterate side by side in 15 to 30 us (3 cases of 101 x 147: 51 us against 19).  Only a clear advantage
-// of the modelled times counts.
+// Whether a batch on the tile engine is faster on chip.  The model of the tile engine's time is 50 us, or 30 and
+// 0.165 per 1000 nodes once its tiles fill the device; a few cases in clusters iterate side by side in 6 to 28 us.
+// Measured with the loop's five overlapped launches, tiles and on chip, us per pseudo-iteration: one case of
+// 51 x 51 45 and 7.6, of 153 x 153 44 and 28; three of 101 x 147 46 and 19; of 153 x 153 7 55 and 28, 8 55 and 55,
+// 15 92 and 83 (left on the tiles), 28 140 and 111, 56 248 and 222, 64 280 and 277, 128 505 and 526; 512 of
+// 51 x 51 358 and 153 (32 x 32 tiles pad small cases); without scalars 64 of 153 x 153 188 and 132, 8 of 200 x 180
+// 59 and 49.  Only a clear advantage of the modelled times counts.
 bool chip_beats_tiles(Batch& b) {
   chip_plan(b);
   double nodes = 0.0;
