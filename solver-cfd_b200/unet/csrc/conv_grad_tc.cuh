@@ -13,6 +13,9 @@
 // tensor memory over the range, the next tile's copies (cp.async) run during the MMAs of this one, and
 // the result is added to the gradient with vector atomics.  A range has at most DW_TILES tiles, so a sum
 // in tensor memory is no longer than about the split-K GEMM's were and the rest is summed in FP32 atomics.
+// Where a tile reaches over the canvas's right edge, tap kx = 0 would multiply the last column of X with the
+// zeros of dZ beyond the edge; that column is cleared before the tap's MMAs, so an infinity or NaN there stays
+// out of a sum that it does not belong to.
 //
 // k_conv_dx: a CTA takes one tile and up to 96 input channels.  Each tap is its own product over the output
 // channels, into one of two accumulators in turn, and is added to the thread's registers while the next
@@ -22,6 +25,8 @@
 // Bound: latency of the short K loops (copies, commits and tensor-memory loads per tap or tile) at two to
 // four CTAs per SM.  Measured: see unet_gemm.cu.
 #pragma once
+#include <type_traits>
+
 #include "conv_tc.cuh"
 
 namespace unet {
@@ -46,12 +51,13 @@ struct DwArgs {
 template <int BN>
 __host__ __device__ constexpr int dw_stage() { return 16 * DW_XPLANE + (BN < 16 ? 16 : BN) / 8 * DW_ZPLANE; }
 
-template <int BN>
+// EDGE: some tiles reach over the right edge (W is not a multiple of CV_W).
+template <int BN, bool EDGE>
 __global__ void __launch_bounds__(TC_THREADS) k_conv_dw(DwArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int STAGE = dw_stage<BN>();
   constexpr int COLS = 3 * BN <= 32 ? 32 : 3 * BN <= 64 ? 64 : 3 * BN <= 128 ? 128 : 3 * BN <= 256 ? 256 : 512;
-  __shared__ unsigned long long bar[2];
+  __shared__ unsigned long long bar[2], edge_bar;
   __shared__ uint32_t tmem_holder;
   __shared__ int wait_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -64,6 +70,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv_dw(DwArgs a) {
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&bar[0]), 1);
     mbar_init(smem_u32(&bar[1]), 1);
+    mbar_init(smem_u32(&edge_bar), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -116,6 +123,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv_dw(DwArgs a) {
   constexpr uint32_t idesc = umma_idesc_mn(TC_BM, BN);
   bool ok = true;
   int last = -1;
+  uint32_t edges = 0;  // tiles at the right edge so far
   for (int t = t0; t < t1; ++t) {
     const int i = t - t0, st = i & 1;
     if (t + 1 < t1) {
@@ -131,16 +139,43 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv_dw(DwArgs a) {
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (threadIdx.x == 0) {
+    const uint32_t sx = s0 + st * STAGE, sz = sx + 16 * DW_XPLANE;
+    const int edge = a.W - t % a.tx * CV_W;  // columns of the canvas from the tile's first on
+    auto issue = [&](auto first, auto end) {  // taps kx from first up to end, by one thread
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint32_t sx = s0 + st * STAGE, sz = sx + 16 * DW_XPLANE;
       for (int k = 0; k < TC_BM / 16; ++k) {  // two rows of 8 pixels per step
         const uint64_t db = umma_desc(sz + k * 256, 128, DW_ZPLANE);
 #pragma unroll
-        for (int kx = 0; kx < 3; ++kx)
+        for (int kx = first.value; kx < end.value; ++kx)
           mma_f16(tmem + kx * BN, umma_desc(sx + (uint32_t)(2 * k * (CV_W + 2) + kx) * 16, (CV_W + 2) * 16, DW_XPLANE), db, idesc,
                   i > 0 || k > 0 ? 1u : 0u);
       }
+    };
+    constexpr std::integral_constant<int, 0> tap0{};
+    constexpr std::integral_constant<int, 1> tap1{};
+    constexpr std::integral_constant<int, 3> tap3{};
+    if (EDGE && edge < CV_W) {
+      if (threadIdx.x == 0) {
+        issue(tap1, tap3);
+        mma_commit(smem_u32(&edge_bar));
+      }
+      ok = cta_wait(smem_u32(&edge_bar), edges & 1u, &wait_flag);
+      ++edges;
+      if (!ok) break;
+      for (int q = threadIdx.x; q < 16 * CV_H; q += TC_THREADS) {  // window column of the canvas's last
+        const int plane = q / CV_H, row = q - plane * CV_H;
+        asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(sx + (uint32_t)(plane * DW_XPLANE + (row * (CV_W + 2) + edge) * 16)),
+                     "r"(0)
+                     : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        issue(tap0, tap1);
+        mma_commit(smem_u32(&bar[st]));
+      }
+    } else if (threadIdx.x == 0) {
+      issue(tap0, tap3);
       mma_commit(smem_u32(&bar[st]));
     }
     last = i;
@@ -150,6 +185,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv_dw(DwArgs a) {
     const bool fin = cta_wait(smem_u32(&bar[last & 1]), (uint32_t)(last >> 1) & 1u, &wait_flag);
     ok = ok && fin;
   }
+  if (EDGE && !ok && edges) cta_wait(smem_u32(&edge_bar), (edges - 1) & 1u, &wait_flag);  // (drains them if it timed out)
   asm volatile("tcgen05.fence::after_thread_sync;");
   if (!ok) {
     if (threadIdx.x == 0 && a.err) atomicExch(a.err, 1);

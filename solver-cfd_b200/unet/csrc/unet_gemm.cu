@@ -115,7 +115,7 @@ cudaError_t conv_bn(const ConvCall& c, int bn) {
 template <int BN>
 cudaError_t dw_go(DwArgs a, cudaStream_t s) {
   const int smem = 2 * dw_stage<BN>();
-  auto k = k_conv_dw<BN>;
+  auto k = a.W % CV_W ? k_conv_dw<BN, true> : k_conv_dw<BN, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   a.nco = (a.N + BN - 1) / BN;
