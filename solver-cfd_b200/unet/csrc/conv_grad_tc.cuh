@@ -20,7 +20,7 @@
 // k_conv_dx: a CTA takes one tile and up to 96 input channels.  Each tap is its own product over the output
 // channels, into one of two accumulators in turn, and is added to the thread's registers while the next
 // tap's MMAs run: the same products and the same order of FP32 additions as the GEMM followed by col2im,
-// so results are bit-identical.
+// so results are bit-identical.  A tap whose pixel lies outside the canvas is not added.
 //
 // Bound: latency of the short K loops (copies, commits and tensor-memory loads per tap or tile) at two to
 // four CTAs per SM.  Measured: see unet_gemm.cu.
@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv_dx(DxArgs a) {
   float s[BN];
 #pragma unroll
   for (int j = 0; j < BN; ++j) s[j] = 0.f;
+  const int m = warp * 32 + lane, mx = x0 + (m & 7), my = y0 + (m >> 3);  // this thread's pixel
   bool ok = true;
   int last = -1;
   // tap's product, once its weights are there (up to `newer` younger copy groups may be in flight)
@@ -298,30 +299,35 @@ __global__ void __launch_bounds__(TC_THREADS) k_conv_dx(DxArgs a) {
     last = tap;
   };
   issue(0, 2);
-  for (int tap = 0; tap < 9; ++tap) {
-    // the next tap's MMAs run while this one's accumulator is read; its TMEM half was read two taps ago
-    if (tap + 1 < 9) issue(tap + 1, tap + 2 < 9 ? 1 : 0);
-    ok = cta_wait(smem_u32(&bar[tap & 1]), (uint32_t)(tap >> 1) & 1u, &wait_flag);
-    if (!ok) break;
-    if (tap + DX_RING < 9) load_w(tap + DX_RING);
-    asm volatile("tcgen05.fence::after_thread_sync;");
+  auto add_taps = [&](auto edge) {
+    for (int tap = 0; tap < 9; ++tap) {
+      // the next tap's MMAs run while this one's accumulator is read; its TMEM half was read two taps ago
+      if (tap + 1 < 9) issue(tap + 1, tap + 2 < 9 ? 1 : 0);
+      ok = cta_wait(smem_u32(&bar[tap & 1]), (uint32_t)(tap >> 1) & 1u, &wait_flag);
+      if (!ok) break;
+      if (tap + DX_RING < 9) load_w(tap + DX_RING);
+      const int ty = my + 1 - tap / 3, tx = mx + 1 - tap % 3;  // the pixel of dZ
+      const bool in = !edge.value || (ty >= 0 && ty < a.H && tx >= 0 && tx < a.W);
+      asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-    for (int n = 0; n < BN; n += 16) {
-      uint32_t r[16];
-      tmem_ld16(r, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((tap & 1) * BN + n));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      for (int n = 0; n < BN; n += 16) {
+        uint32_t r[16];
+        tmem_ld16(r, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((tap & 1) * BN + n));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int j = 0; j < 16; ++j) s[n + j] += __uint_as_float(r[j]);
+        for (int j = 0; j < 16; ++j) s[n + j] = in ? s[n + j] + __uint_as_float(r[j]) : s[n + j];
+      }
     }
-  }
+  };
+  if (x0 > 0 && y0 > 0 && x0 + CV_W < a.W && y0 + CV_H < a.H) add_taps(std::false_type{});
+  else add_taps(std::true_type{});
   asm volatile("cp.async.wait_all;" ::: "memory");
   if (!ok) {  // one more bounded wait drains the MMAs issued (see k_gemm_tc)
     cta_wait(smem_u32(&bar[last & 1]), (uint32_t)(last >> 1) & 1u, &wait_flag);
     if (threadIdx.x == 0 && a.err) atomicExch(a.err, 1);
   } else {
-    const int m = warp * 32 + lane, x = x0 + (m & 7), y = y0 + (m >> 3);
-    if (x < a.W && y < a.H) {
-      float* d = a.dX + (((long long)b * a.H + y) * a.W + x) * a.C + ci0;
+    if (mx < a.W && my < a.H) {
+      float* d = a.dX + (((long long)b * a.H + my) * a.W + mx) * a.C + ci0;
       const int n1 = a.C - ci0;
       if ((a.C & 3) == 0) {
 #pragma unroll

@@ -2,6 +2,7 @@
 import pytest
 
 from test_unet_conv import L  # noqa: F401 - fixture
+from test_unet_kernels import _gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -34,5 +35,34 @@ def test_dw_with_infinities_and_nan(L, B, H, W, Cin, Cout):  # noqa: F811
         assert L.unet_im2col(X.data_ptr(), B, H, W, Cin, kp, col.data_ptr(), None) == 0
         bad = ~torch.isfinite(col.float()).all(0)
         assert torch.equal(~torch.isfinite(gw), bad[:, None].expand(kp, Cout)), (y, x)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+
+
+@SIZES
+@pytest.mark.parametrize("where", ["weight", "dz"])
+def test_dx_with_infinities_and_nan(L, B, H, W, Cin, Cout, where):  # noqa: F811
+    """The same for dX: the values that the GEMM and col2im give."""
+    import torch
+    if not L.unet_conv3x3_dx_fits(Cin, Cout):
+        pytest.skip("dX of these channels goes through col2im")
+    g = torch.Generator(device="cuda").manual_seed(W)
+    M, kp = B * H * W, (9 * Cin + 7) // 8 * 8
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for q, y, x, v in _places(H, W):
+        dz = torch.randn(M, Cout, device="cuda", generator=g).to(torch.bfloat16)
+        Wt = torch.randn(kp, Cout, device="cuda", generator=g).to(torch.bfloat16)
+        if where == "weight":
+            Wt[q * Cin + 1, q % Cout] = v  # of tap q
+        else:
+            dz[y * W + x, q % Cout] = v
+        dcol = torch.zeros(M, kp, device="cuda")
+        d0 = torch.zeros(M, Cin, device="cuda")
+        d1 = torch.zeros_like(d0)
+        assert _gemm(L, dz, Wt, M, kp, Cout, 0, Cbuf=dcol) == 0
+        assert L.unet_col2im(dcol.data_ptr(), B, H, W, Cin, kp, d0.data_ptr(), None) == 0
+        assert L.unet_conv3x3_dx(dz.data_ptr(), Wt.data_ptr(), B, H, W, Cin, Cout, d1.data_ptr(), err.data_ptr(), None) == 0
+        assert torch.equal(torch.isfinite(d0), torch.isfinite(d1)), (y, x)
+        assert torch.equal(torch.nan_to_num(d0), torch.nan_to_num(d1)), (y, x)
     torch.cuda.synchronize()
     assert int(err.item()) == 0
