@@ -32,8 +32,9 @@
 // k_control to the arrays.  Every iteration runs the same kernels and arithmetic.
 //
 // Launches: the five kernels of an iteration are chained by programmatic dependent launch, so a kernel's
-// CTAs start while the last ones of the kernel before it finish (64 cases at 153 x 153: 297.9 -> 294.0 us per
-// pseudo-iteration with transfers, 1024 x 512: 104.6 -> 103.1).
+// CTAs start while the last ones of the kernel before it finish.  Measured against seven launches in order, us per
+// pseudo-iteration: 64 cases of 153 x 153 276.4 -> 274.2, 1024 x 512 99.4 -> 98.8; k_te_uv<2> by itself, which
+// now carries the passes above, 53.4 -> 54.2 (55.4 while it loaded tau_dirty only when its boxes had arrived).
 //
 // TMA: 2-D tensor maps over each case buffer (dims pitch x (ny+1), FP64, no swizzle, zero fill
 // outside), non-multicast loads into 128-byte aligned shared memory, one mbarrier per CTA with the
@@ -356,6 +357,7 @@ __global__ void __launch_bounds__(TE_THREADS, 2) k_te_uv(const CaseDev* __restri
   // the buoyancy factor w = 1 - 2/(T(i,j) + T(i,j-1)) of the physical-step temperature: stage 1 of
   // a step's first pseudo-iteration computes it from T and stores it, every other launch loads it
   const bool fresh = ST == 1 && kc->k == 0;
+  const bool dirty = ST > 1 && kc->tau_dirty != 0;
 
   double* Ub = reinterpret_cast<double*>(sm);  // um_tau box
   double* Vb = Ub + BU * BU;                   // vm_tau box
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(TE_THREADS, 2) k_te_uv(const CaseDev* __restri
     __syncthreads();
     Vs = Vc;
   }
-  if (ST > 1 && kc->tau_dirty && (t.i0 - 2 <= 2 || t.i0 + NT + 1 >= nx || t.j0 - 2 <= 2 || t.j0 + NT + 1 >= ny)) {
+  if (dirty && (t.i0 - 2 <= 2 || t.i0 + NT + 1 >= nx || t.j0 - 2 <= 2 || t.j0 + NT + 1 >= ny)) {
     // the first iteration after an upload: stages 2 and 3 read um_tau and vm_tau after the boundary
     // passes (the arrays themselves are rewritten by k_control)
     const Win wu{Ub, t.i0 - 2, t.j0 - 2, BU, BU, BU}, wv{Vb, t.i0 - 2, t.j0 - 2, BU, BU, BU};
