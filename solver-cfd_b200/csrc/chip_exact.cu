@@ -38,7 +38,6 @@ __device__ __forceinline__ double pos_part(double a) { return a > 0.0 ? a : 0.0;
 __device__ __noinline__ double plain_quotient(double a, double b) { return a / b; }
 
 struct ChipExact {
-  static constexpr bool EXACT = true;
   enum { K_IPHI, K_E1RE, K_EPRE, K_REDA, K_IREDA, K_CFS, K_KT, K_KC, K_CAP, K_ICAP };
   // constants of the case, each the value that the reference's expression has
   static __device__ void constants(const CaseDev& d, double* k) {

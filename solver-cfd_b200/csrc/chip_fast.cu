@@ -13,7 +13,6 @@ __device__ __forceinline__ double face(const FaceK& k, double f, double up2, dou
 }
 
 struct ChipFast {
-  static constexpr bool EXACT = false;
   static __device__ void constants(const CaseDev&, double*) {}
   static __device__ __forceinline__ double buoy(const ChipCtx&, double T0, double T1) { return 1.0 - 2.0 / (T0 + T1); }
   // RESU and RESV at a node: U, V the stage inputs, ut, vt the tau arrays, p the pressure, each at the

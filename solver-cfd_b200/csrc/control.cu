@@ -102,17 +102,15 @@ __global__ void k_control(const CaseDev* __restrict__ cs, CaseCtl* __restrict__ 
       }
       if (k.active) atomicAdd(n_active, 1);
     }
-    if (end.mode != LOOP_NONE) {
-      // the block that finishes last counts the iteration and decides whether another follows
+    // the block that finishes last counts the iteration and decides whether another follows
+    __threadfence();
+    if (atomicAdd(end.ticket, 1) == (int)gridDim.x - 1) {
       __threadfence();
-      if (atomicAdd(end.ticket, 1) == (int)gridDim.x - 1) {
-        __threadfence();
-        *end.ticket = 0;
-        const int a = atomicExch(n_active, 0);
-        const long long it = ++*end.iter_count;
-        if (end.mode == LOOP_COND) cudaGraphSetConditional(end.handle, (a > 0 && it < end.max_iters) ? 1u : 0u);
-        else *(volatile int*)end.host_flag = a;
-      }
+      *end.ticket = 0;
+      const int a = atomicExch(n_active, 0);
+      const long long it = ++*end.iter_count;
+      if (end.mode == LOOP_COND) cudaGraphSetConditional(end.handle, (a > 0 && it < end.max_iters) ? 1u : 0u);
+      else *(volatile int*)end.host_flag = a;
     }
   }
   __syncthreads();

@@ -25,7 +25,7 @@ cudaError_t launch_cell_fields(const double* um, const double* vm, int nx, int n
                                double* mag, cudaStream_t s);
 
 // loop control (control.cu)
-enum LoopMode { LOOP_NONE = 0, LOOP_COND = 1, LOOP_FLAG = 2 };
+enum LoopMode { LOOP_COND = 1, LOOP_FLAG = 2 };
 struct LoopEnd {
   int mode;                           // what the last block does with the number of active cases
   int tau_bc;                         // 1: apply the first iteration's side effects on um_tau, vm_tau
