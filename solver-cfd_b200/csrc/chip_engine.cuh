@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(CHIP_THREADS, 1) k_chip(ChipArgs a) {
       uv_stage(ph, doU, doV, U(in), V(in), U(out), V(out), U(ut), V(ut), Pw(rp_read));
     }
     if ((z || ph == 4) && has) {
-      const int nu = ph == 4 || fin == EXIT ? ua : ut;  // the velocities of the iteration that T, C belong to
+      const int nu = ph == 4 || fin == EXIT || fin == FAILED ? ua : ut;  // the velocities of the iteration that T, C belong to
       tc_stage(z, z != 1 || t_made, U(nu), V(nu), Tw(zi), Cw(zi), Tw(zo), Cw(zo), Tw(tt), Cw(tt), Pw(rp0), ph == 4 ? pn : nullptr);
     }
     if (ph == 4) {
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(CHIP_THREADS, 1) k_chip(ChipArgs a) {
       total += 1;
       if (e != e || e > 1.0e300) {
         fin = FAILED;
-        pend = false;
+        pend = scal && a.tc_of_failed;
       } else if (itc != 1 && e < d.eps) {
         fin = EXIT;
       } else {
@@ -689,6 +689,12 @@ __global__ void __launch_bounds__(CHIP_THREADS, 1) k_chip(ChipArgs a) {
       active = false;
       store_rows(d.U[g.ru[R_NTAU]], U(ua));
       store_rows(d.V[g.rv[R_NTAU]], V(ua));
+      if (ph == 6) {
+        finish_c(Tw(ta), false, d.T_in);
+        finish_c(Cw(ta), false, d.C_in);
+        store_rows(d.T[g.rt[R_NTAU]], Tw(ta));
+        store_rows(d.C[g.rc[R_NTAU]], Cw(ta));
+      }
     } else {
       // EXIT: the tau copies are skipped and the new iterate becomes the physical-step state (its buffer
       // and n_tau's change roles); CAP: the loop condition failed after the copies, phys = latest iterate

@@ -24,6 +24,7 @@ struct ChipArgs {
   int* iters;        // [case * n_steps + step]
   double* err;
   int corner_role;   // role of the vm buffer whose history gives vm(imax, jmax+1) (see k_chip)
+  bool tc_of_failed;  // a failed case's T and C n_tau arrays get the failing iteration's values (tile engine)
 };
 
 // Shared-memory layout of one CTA, offsets in doubles, the same in every CTA of a cluster: strips of

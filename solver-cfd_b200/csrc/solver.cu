@@ -1107,7 +1107,7 @@ int run_engine(Batch& b) {
       const bool phys = (cls / 17 - 1) & 1, quick = (cls / 17 - 1) & 2;
       size_t smem = 0;
       for (int q = 0; q < cnt; ++q) smem = std::max(smem, chip_bytes(plan_case(b, order[off + q]), K, phys));
-      ChipArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err, b.engine == 2 ? R_PHYS : R_NTAU};
+      ChipArgs a{b.dc, b.dk, b.d_cases + off, b.d_iters, b.d_err, b.engine == 2 ? R_PHYS : R_NTAU, b.engine == 2};
       e = (b.use_fast ? launch_chip_fast : launch_chip_exact)(a, K, cnt, phys, quick, smem, s);
     } else {
     // staging slot: the largest strip of the size class plus two halo rows on each side

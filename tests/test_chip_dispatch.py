@@ -89,3 +89,62 @@ def test_loop_kind_does_not_choose_kernels(gpu, monkeypatch, n, nx, ny, used):
         b.close()
     for k in outs[0]:
         assert np.array_equal(outs[0][k], outs[1][k]), k
+
+
+def _ends(pkg):
+    """Cases, a value put into one field, and runs: steps that end at itc_max, by the exit test (also in the
+    first iterations), and with a residual that is NaN or infinite, from each field that can cause it."""
+    cfg = pkg.configs
+    full = dict(arith=pkg.ARITH_FAST)
+    ref = lambda **kw: cfg.reference_case(12, arith=pkg.ARITH_FAST, **kw)[:4]  # noqa: E731
+    plain = cfg.channel_case(45, 33, seed=4, Re=100.0, scheme=pkg.SCHEME_UPWIND, itc_max=40, arith=pkg.ARITH_FAST)
+    capped = _item(pkg, 40, 30, itc_max=50, **full)
+    return {
+        "cap": (capped, None, [(2, 1), (1, 0)]),
+        "exit": (_item(pkg, 30, 22, itc_max=3000, eps=3e-2, **full), None, [(3, 1), (2, 0)]),
+        "exit-at-once": (_item(pkg, 30, 22, itc_max=3000, eps=1e3, **full), None, [(3, 1), (2, 0)]),
+        "nan": (capped, ("um_tau", np.nan), [(3, 1)]),
+        "overflow": (capped, ("vm", 1e150), [(3, 1)]),
+        "T-inf": (capped, ("T", np.inf), [(3, 1)]),
+        "C-nan": (capped, ("C_tau", np.nan), [(3, 1)]),
+        "T-zero": (capped, ("T", 0.0), [(2, 1)]),
+        "plain-cap": (plain, None, [(2, 1), (1, 0)]),
+        "plain-p-inf": (plain, ("p", np.inf), [(2, 1)]),
+        "plain-pn-nan": (plain, ("pn", np.nan), [(2, 1)]),
+        "reference-cap": (ref(itc_max=40), None, [(2, 1), (1, 0)]),
+        "reference-exit": (ref(itc_max=4000, eps=3e-3), None, [(4, 1), (2, 0)]),
+        "reference-nan": (ref(itc_max=40), ("um", np.nan), [(2, 1)]),
+    }
+
+
+@pytest.mark.parametrize("engine", [0, 2], ids=["cluster", "tile"])
+@pytest.mark.parametrize("end", ["cap", "exit", "exit-at-once", "nan", "overflow", "T-inf", "C-nan", "T-zero", "plain-cap",
+                                 "plain-p-inf", "plain-pn-nan", "reference-cap", "reference-exit", "reference-nan"])
+def test_on_chip_ends_like_the_engine_it_stands_in_for(gpu, engine, end):
+    """FAST arithmetic, on chip and off: the same counts and status, every one of the 14 fields within 1e-10 of its
+    largest value (the bound of the FAST engines) and with infinities and NaN at the same nodes, whatever
+    ended the run."""
+    from conftest import mask_dead
+    (prm, mesh, st, itc), kick, runs = _ends(gpu)[end]
+    st = {k: v.copy(order="F") for k, v in st.items()}
+    if kick:
+        st[kick[0]][5, 7] = kick[1]
+    got = []
+    for off in (0, 1):
+        b = gpu.Batch([prm], [mesh])
+        b.set_option(gpu.OPT_ENGINE, engine)
+        b.set_option(gpu.OPT_ON_CHIP, off)
+        b.set_state(0, st)
+        log = [b.run(n, [i]) for n, i in runs]
+        assert b.engines_used() == ((gpu.USED_TILE if engine else gpu.USED_CLUSTER) if off else gpu.USED_CHIP)
+        got.append((log, b.get_state(0)))
+        b.close()
+    for x, y in zip(got[0][0], got[1][0]):
+        for k in (0, 1, 3):
+            assert np.array_equal(x[k], y[k])
+        assert np.allclose(x[2], y[2], rtol=1e-9, atol=0.0, equal_nan=True)
+    for k in got[0][1]:
+        x, y = (mask_dead(k, g[1][k], prm.bc) for g in got)
+        ok = np.isfinite(y)
+        assert np.array_equal(np.isfinite(x), ok), k
+        assert not ok.any() or np.abs(x[ok] - y[ok]).max() <= 1e-10 * np.abs(y[ok]).max(), k
