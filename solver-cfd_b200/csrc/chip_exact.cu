@@ -6,8 +6,8 @@
 //   * a quotient by a metric difference, a porosity or another constant of the case is computed from
 //     the constant's correctly rounded reciprocal (exact_div), five dependent FP64 instructions instead
 //     of a division routine of about 114 cycles;
-//   * a quotient by a porosity of 1 and the drag of a node without porous structure (a product with 0)
-//     are left out.
+//   * a quotient by a porosity of 1 and, unless it has overflowed, the drag of a node without porous
+//     structure (a product with 0) are left out.
 // Reference (OpenMp_Multicore/): RESU equations.f90:2-116 (+ upwind_Ui/Uj :120-240), RESV :305-420
 // (+ upwind_Vi/Vj :423-542), solve_P :607-665, RESZ :723-765, RESC :823-867.
 #include "chip_engine.cuh"
@@ -92,13 +92,17 @@ struct ChipExact {
     c = quo<SAFE>(c, x.d.phi, x.k[K_IPHI], bad);
     e = quo<SAFE>(e, x.d.phi, x.k[K_IPHI], bad);
   }
-  // r minus the Darcy-Forchheimer drag of velocity a at a node with velocity (u, v)
+  // r minus the Darcy-Forchheimer drag of velocity a at a node with velocity (u, v).  Without porous structure
+  // the reference multiplies the drag with liga = 0: nothing, or NaN where it has overflowed, which takes
+  // u*u + v*v above 2^600 (chip_divisors and Cf); such a node is computed in full.
   template <bool SAFE>
   static __device__ __forceinline__ double drag(const ChipCtx& x, double r, double a, double u, double v, bool por, bool& bad) {
     const double s = u * u + v * v;
     if (por)
       return r - x.d.phi * (quo<SAFE>(a, x.k[K_REDA], x.k[K_IREDA], bad) + x.k[K_CFS] * a * sqrt(s)) * 1.0;
-    return r - s * 0.0;  // the reference's product with liga = 0: 0, or NaN once s has overflowed
+    if (SAFE) return r - 1.0 * (a / x.k[K_REDA] + x.d.Cf / sqrt(1.0 * x.d.Da) * a * sqrt(s)) * 0.0;
+    bad |= (unsigned)__double2hiint(s) >= (1023u + 600u) << 20;
+    return r;
   }
   // RESU and RESV at a node: U, V the stage inputs, ut, vt the tau arrays, p the pressure, each at the
   // node (neighbours at +-1 and +-P)

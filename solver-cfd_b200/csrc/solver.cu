@@ -238,7 +238,8 @@ bool binary_porosity(const acs_grid& g, double* phi) {
 // constants must be positive and far from the exponent limits.
 bool chip_divisors(const acs_grid& g, const acs_params& p, double phi) {
   auto ok = [](double v) { return v >= 0x1p-60 && v <= 0x1p60; };
-  bool r = ok(phi) && ok(1.0 * (phi - 1.0) + 1.0) && ok(p.Re * p.Da) && ok(p.Re) && ok(p.Pe) && ok(p.Re * p.Sc);
+  bool r = ok(phi) && ok(1.0 * (phi - 1.0) + 1.0) && ok(p.Re * p.Da) && ok(p.Re) && ok(p.Pe) && ok(p.Re * p.Sc) &&
+           std::fabs(p.Cf) <= 0x1p200;
   for (int i = 1; i < g.imax; ++i) r = r && ok(g.x[i] - g.x[i - 1]);
   for (int j = 1; j < g.jmax; ++j) r = r && ok(g.y[j] - g.y[j - 1]);
   for (int i = 2; i < g.imax; ++i) r = r && ok(g.xm[i] - g.xm[i - 1]);  // interior cells only
