@@ -66,3 +66,36 @@ def test_dx_with_infinities_and_nan(L, B, H, W, Cin, Cout, where):  # noqa: F811
         assert torch.equal(torch.nan_to_num(d0), torch.nan_to_num(d1)), (y, x)
     torch.cuda.synchronize()
     assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("where", ["x", "weight"])
+@pytest.mark.parametrize("B,H,W,Cin,Cout", [(1, 20, 20, 32, 40), (2, 18, 13, 11, 16), (1, 33, 9, 144, 136)])
+def test_forward_with_infinities_and_nan(L, B, H, W, Cin, Cout, where):  # noqa: F811
+    """The same for the convolution itself (window and gathering kernel): the values of im2col and the GEMM."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(W)
+    M, kp = B * H * W, (9 * Cin + 7) // 8 * 8
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for q, y, x, v in _places(H, W):
+        X = torch.randn(M, Cin, device="cuda", generator=g).to(torch.bfloat16)
+        Wt = torch.randn(Cout, kp, device="cuda", generator=g).to(torch.bfloat16)
+        Wt[:, 9 * Cin:] = 0.0
+        if where == "x":
+            X[y * W + x, q % Cin] = v
+        else:
+            Wt[q % Cout, q * Cin + 1] = v  # of tap q
+        col = torch.zeros(M, kp, dtype=torch.bfloat16, device="cuda")
+        y0 = torch.zeros(M, Cout, dtype=torch.bfloat16, device="cuda")
+        y1 = torch.zeros_like(y0)
+        assert L.unet_im2col(X.data_ptr(), B, H, W, Cin, kp, col.data_ptr(), None) == 0
+        assert _gemm(L, col, Wt, M, Cout, kp, 2, Y=y0) == 0
+        if Cin % 16 == 0:
+            assert L.unet_conv3x3(X.data_ptr(), B, H, W, Cin, Wt.data_ptr(), kp, Cout, 2, None, y1.data_ptr(), Cout, None, 0,
+                                  err.data_ptr(), None) == 0
+        else:
+            assert L.unet_conv3x3_gather(X.data_ptr(), B, H, W, Cin, Wt.data_ptr(), kp, kp, Cout, y1.data_ptr(), Cout, None, 0,
+                                         err.data_ptr(), None) == 0
+        assert torch.equal(torch.isfinite(y0), torch.isfinite(y1)), (y, x)
+        assert torch.equal(torch.nan_to_num(y0.float()), torch.nan_to_num(y1.float())), (y, x)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
