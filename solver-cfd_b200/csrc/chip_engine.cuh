@@ -18,8 +18,8 @@
 // Bound: latency.  Four empty phases take 2.3 us of a pseudo-iteration (a cluster barrier alone 0.22 us
 // with 256 threads), a node's loads, address arithmetic and dependence chain most of the rest; the FP64
 // pipe (one warp instruction per two clocks and SM quarter) is busy for a fifth to a third of the time.
-// Measured on one B200, us per pseudo-iteration, cluster engine -> this engine: 51 x 84 EXACT 208 -> 16.5,
-// 51 x 51 upwind FAST 34 -> 5.6, 102 x 102 full FAST 64 -> 15.0, 8 cases of 153 x 153 EXACT 394 -> 112.
+// Measured on one B200, us per pseudo-iteration, cluster engine -> this engine: 51 x 84 EXACT 208 -> 16.6,
+// 51 x 51 upwind FAST 34 -> 5.4, 102 x 102 full FAST 64 -> 14.7, 8 cases of 153 x 153 EXACT 394 -> 99.
 //
 // Termination: as in engine.cuh -- identical decisions from identical residuals in every CTA, at most
 // itc_max iterations per step.
