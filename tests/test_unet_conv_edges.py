@@ -99,3 +99,44 @@ def test_forward_with_infinities_and_nan(L, B, H, W, Cin, Cout, where):  # noqa:
         assert torch.equal(torch.nan_to_num(y0.float()), torch.nan_to_num(y1.float())), (y, x)
     torch.cuda.synchronize()
     assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 1, 1), (3, 1, 2), (2, 2, 1), (1, 17, 9), (70, 3, 5)])
+@pytest.mark.parametrize("Cin,Cout", [(16, 8), (11, 16), (32, 32), (3, 64)])
+def test_tiny_canvases(L, B, H, W, Cin, Cout):  # noqa: F811
+    """Canvases smaller than a tile, and just larger: the convolution and dX bit-identical to im2col, GEMM and
+    col2im, dW within 2e-6 of the FP64 product's norm (at most 1050 products per sum, FP32)."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(H * W + Cin)
+    M, kp = B * H * W, (9 * Cin + 7) // 8 * 8
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    X = torch.randn(M, Cin, device="cuda", generator=g).to(torch.bfloat16)
+    dz = torch.randn(M, Cout, device="cuda", generator=g).to(torch.bfloat16)
+    Wt = torch.randn(Cout, kp, device="cuda", generator=g).to(torch.bfloat16)
+    Wt[:, 9 * Cin:] = 0.0
+    wt = Wt.t().contiguous()
+    col = torch.zeros(M, kp, dtype=torch.bfloat16, device="cuda")
+    y0 = torch.zeros(M, Cout, dtype=torch.bfloat16, device="cuda")
+    y1 = torch.zeros_like(y0)
+    assert L.unet_im2col(X.data_ptr(), B, H, W, Cin, kp, col.data_ptr(), None) == 0
+    assert _gemm(L, col, Wt, M, Cout, kp, 2, Y=y0) == 0
+    if Cin % 16 == 0:
+        assert L.unet_conv3x3(X.data_ptr(), B, H, W, Cin, Wt.data_ptr(), kp, Cout, 2, None, y1.data_ptr(), Cout, None, 0,
+                              err.data_ptr(), None) == 0
+    else:
+        assert L.unet_conv3x3_gather(X.data_ptr(), B, H, W, Cin, Wt.data_ptr(), kp, kp, Cout, y1.data_ptr(), Cout, None, 0,
+                                     err.data_ptr(), None) == 0
+    assert torch.equal(y0, y1)
+    gw = torch.zeros(kp, Cout, device="cuda")
+    assert L.unet_conv3x3_dw(X.data_ptr(), dz.data_ptr(), B, H, W, Cin, Cout, gw.data_ptr(), err.data_ptr(), None) == 0
+    ref = col.double().t() @ dz.double()
+    assert float((gw.double() - ref).norm()) <= 2e-6 * float(ref.norm())
+    dcol = torch.zeros(M, kp, device="cuda")
+    d0 = torch.zeros(M, Cin, device="cuda")
+    d1 = torch.full((M, Cin), float("nan"), device="cuda")
+    assert _gemm(L, dz, wt, M, kp, Cout, 0, Cbuf=dcol) == 0
+    assert L.unet_col2im(dcol.data_ptr(), B, H, W, Cin, kp, d0.data_ptr(), None) == 0
+    assert L.unet_conv3x3_dx(dz.data_ptr(), wt.data_ptr(), B, H, W, Cin, Cout, d1.data_ptr(), err.data_ptr(), None) == 0
+    assert torch.equal(d0, d1)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
