@@ -253,7 +253,10 @@ int flush_ctl(Batch& b);
 // Whether a caller is capturing the batch's stream.
 bool capturing(const Batch& b) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(b.stream, &st) != cudaSuccess) cudaGetLastError();
+  if (cudaStreamIsCapturing(b.stream, &st) != cudaSuccess) {  // (the legacy stream, while another one is captured)
+    cudaGetLastError();
+    return false;
+  }
   return st != cudaStreamCaptureStatusNone;
 }
 
